@@ -7,10 +7,18 @@
 
 namespace yg {
 
+static PoleSet one_pole(const double *lhs, const double *rhs, double w) {
+  PoleSet ps{};
+  ps.n = 1;
+  ps.lhs[0] = (const double2 *)lhs;
+  ps.rhs[0] = (const double2 *)rhs;
+  ps.w[0] = w;
+  return ps;
+}
+
 void clover_fermion_force(Lattice &L, double residue, double *lhs, double *rhs) {
   if (!L.p.clover) return;
-  YG_DISPATCH_D(L.d, K::clover_fermion_force(L.cl_force.as<double2>(), (const double2 *)lhs, (const double2 *)rhs,
-                                             L.g, residue, L.stream));
+  YG_DISPATCH_D(L.d, K::clover_fermion_force(L.cl_force.as<double2>(), one_pole(lhs, rhs, residue), L.g, L.stream));
   YG_LAUNCHED();
 }
 
@@ -27,8 +35,8 @@ void wilson_fermion_force(Lattice &L, double dt, double mass, double residue, do
     coeff = -coeff;
   }
   if (L.p.clover) clover_fermion_force(L, residue, lhs, rhs);
-  YG_DISPATCH_D(L.d, K::hopping_force(L.mom.as<double>(), (const double2 *)lhs, (const double2 *)rhs,
-                                      L.links.as<double2>(), L.g, L.rt.itrepr, L.ng, coeff, L.stream));
+  YG_DISPATCH_D(L.d, K::hopping_force(L.mom.as<double>(), one_pole(lhs, rhs, coeff), L.links.as<double2>(), L.g,
+                                      L.rt.itrepr, L.ng, L.stream));
   YG_LAUNCHED();
 }
 
@@ -68,12 +76,12 @@ void wilson_fermion_force_q_multi(Lattice &L, double dt, double mass, int n, con
   }
   if (L.p.clover) {
     for (int k = 0; k < n; k++) ps.w[k] = residue[k];
-    YG_DISPATCH_D(L.d, K::clover_fermion_force_multi(L.cl_force.as<double2>(), ps, L.g, L.stream));
+    YG_DISPATCH_D(L.d, K::clover_fermion_force(L.cl_force.as<double2>(), ps, L.g, L.stream));
     YG_LAUNCHED();
   }
   for (int k = 0; k < n; k++) ps.w[k] = (L.p.eo ? -1.0 : 1.0) * dt * residue[k];
-  YG_DISPATCH_D(L.d, K::hopping_force_multi(L.mom.as<double>(), ps, L.links.as<double2>(), L.g, L.rt.itrepr, L.ng,
-                                            L.stream));
+  YG_DISPATCH_D(L.d, K::hopping_force(L.mom.as<double>(), ps, L.links.as<double2>(), L.g, L.rt.itrepr, L.ng,
+                                      L.stream));
   YG_LAUNCHED();
 }
 
@@ -85,7 +93,7 @@ void begin_fermion_force(Lattice &L) {
 void clover_logdet_force(Lattice &L, double mass, double residue) {
   if (!L.p.clover) return;
   ensure_ldl(L, 4.0 + mass);
-  YG_DISPATCH_D(L.d, K::clover_ldl_force(L.cl_force.as<double2>(), L.ldl.as<double2>(), L.g, residue, L.stream));
+  YG_DISPATCH_D(L.d, K::clover_ldl_force(L.cl_force.as<double2>(), L.cpk64.as<double2>(), L.g, residue, L.stream));
   YG_LAUNCHED();
 }
 

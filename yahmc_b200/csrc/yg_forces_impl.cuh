@@ -59,6 +59,15 @@ __device__ __forceinline__ void g5_omg(double2 (&o)[4][D], const double2 (&s)[4]
   }
 }
 
+template <int D>
+__device__ __forceinline__ void scale_spinor(double2 (&s)[4][D], double w) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    YG_UNROLL_DF
+    for (int c = 0; c < D; c++) s[k][c] = cscale(s[k][c], w);
+  }
+}
+
 // fmat[i][j] += sum_k a[k][i] conj(b[k][j])  (fmat_create, forces.cpp:13-30)
 template <int D>
 __device__ __forceinline__ void outer_acc(double2 (&f)[D * D], const double2 (&a)[4][D], const double2 (&b)[4][D]) {
@@ -119,9 +128,181 @@ __device__ __forceinline__ void dag(double2 (&c)[D * D], const double2 (&a)[D * 
   }
 }
 
-// ---- clover_fermion_force, forces.cpp:122-172 (all sites)
+// X <- M X (DAG: M^dag X) for the matrix M of record (id, slot), in place column by column: the
+// chains of products below are written as such left multiplications, so that a thread holds the
+// running product, one sum and one loaded matrix, and d = 3 stays within 168 registers
+template <int D, bool DAG>
+__device__ __forceinline__ void lmul(double2 (&X)[D * D], const double2 *base, const Geom &g, int id, int slot,
+                                     int nslots) {
+  double2 M[D * D];
+  asm volatile("" ::: "memory");     // M's loads stay behind the previous product: hoisting them all costs spills
+  ld_mat<D>(M, base, g, id, slot, nslots);
+  YG_UNROLL_DF
+  for (int j = 0; j < D; j++) {
+    double2 v[D];
+    YG_UNROLL_DF
+    for (int i = 0; i < D; i++) {
+      double2 t = make_double2(0, 0);
+      YG_UNROLL_DF
+      for (int k = 0; k < D; k++) {
+        if (DAG) cfmac(t, M[k * D + i], X[k * D + j]);
+        else cfma(t, M[i * D + k], X[k * D + j]);
+      }
+      v[i] = t;
+    }
+    YG_UNROLL_DF
+    for (int i = 0; i < D; i++) X[i * D + j] = v[i];
+  }
+}
+
+// t += M X
 template <int D>
-__global__ void k_clover_fermion_force(double2 *clf, const double2 *lhs, const double2 *rhs, Geom g, double residue) {
+__device__ __forceinline__ void lmul_add(double2 (&t)[D * D], const double2 (&X)[D * D], const double2 *base,
+                                         const Geom &g, int id, int slot, int nslots) {
+  double2 M[D * D];
+  asm volatile("" ::: "memory");
+  ld_mat<D>(M, base, g, id, slot, nslots);
+  YG_UNROLL_DF
+  for (int i = 0; i < D; i++) {
+    YG_UNROLL_DF
+    for (int j = 0; j < D; j++) {
+      YG_UNROLL_DF
+      for (int k = 0; k < D; k++) cfma(t[i * D + j], M[i * D + k], X[k * D + j]);
+    }
+  }
+}
+
+// out[a * OST] = coeff/(-TF) * Re tr(iT[a] m) (algebra_project, suNa.cpp:91-111), TF = 2.  The
+// colour loops are unrolled for d <= 4, so that m stays in registers; every lane reads the same
+// generator entries.
+template <int D, int OST>
+__device__ __forceinline__ void project_store(double *out, const double2 (&m)[D * D], const double2 *gens, int ng,
+                                              double coeff) {
+  const double c = coeff / -2.0;
+#pragma unroll 1
+  for (int a = 0; a < ng; a++) {
+    double tr = 0;
+    const double2 *t = gens + a * D * D;
+    YG_UNROLL_DF
+    for (int i = 0; i < D; i++) {
+      YG_UNROLL_DF
+      for (int k = 0; k < D; k++) {
+        const double2 w = __ldg(t + i * D + k), v = m[k * D + i];
+        tr = fma(w.x, v.x, fma(-w.y, v.y, tr));
+      }
+    }
+    out[a * OST] = c * tr;
+  }
+}
+
+// Force kernels take 32 consecutive sites per block, lane = site, so that every field, link and
+// cl_force access of a warp is a contiguous run, with one warp per direction (and plane).  The
+// per-link algebra components go through shared memory: acc[(warp * ng + a) * 33 + lane]
+// (a stride of 33 doubles), NW warps per direction summed in order, then the block adds its
+// 32 sites x NMU directions of momenta (the AoS records [site][mu][a]) in one coalesced pass.
+template <int NMU, int NW>
+__device__ __forceinline__ void add_momenta(double *mom, const double *acc, const Geom &g, int site0, int mu0, int ng) {
+  __syncthreads();
+  for (int e = threadIdx.x; e < 32 * NMU * ng; e += blockDim.x) {
+    const int a = e % ng, mu = (e / ng) % NMU, lane = e / (ng * NMU);
+    if (site0 + lane >= g.V) continue;
+    double v = 0;
+#pragma unroll
+    for (int w = 0; w < NW; w++) v += acc[((mu * NW + w) * ng + a) * 33 + lane];
+    mom[((long)(site0 + lane) * 4 + mu0 + mu) * ng + a] += v;
+  }
+}
+
+constexpr size_t momenta_smem(int warps, int ng) { return sizeof(double) * 33 * warps * ng; }
+
+// ---- clover_fermion_force, forces.cpp:122-172 (all sites), summed over the poles of a
+// rational approximation (rhmc.cpp:86-106 calls wilson_fermion_force_q once per pole; one pole
+// is the plain force): cl_force is read and written once, 1728 B a site for d = 3, which bounds it.
+// fmat of one slot and the poles, added to cl_force
+template <int D>
+__device__ __forceinline__ void clover_slot_force(double2 *clf, const PoleSet &ps, const Geom &g, int id, int slot) {
+  double2 f[D * D];
+  YG_UNROLL_DF
+  for (int k = 0; k < D * D; k++) f[k] = make_double2(0, 0);
+#pragma unroll 1
+  for (int n = 0; n < ps.n; n++) {
+    double2 l[4][D], r[4][D], s[4][D];
+    ld_spinor64<D>(l, ps.lhs[n], g, id);
+    ld_spinor64<D>(r, ps.rhs[n], g, id);
+    g5_sigma<D>(s, l, slot);
+    scale_spinor<D>(s, ps.w[n]);
+    outer_acc<D>(f, s, r);
+    g5_sigma<D>(s, r, slot);
+    scale_spinor<D>(s, ps.w[n]);
+    outer_acc<D>(f, s, l);
+  }
+  YG_UNROLL_DF
+  for (int k = 0; k < D * D; k++) {
+    long ix = fidx(g, id, slot * D * D + k, 6 * D * D);
+    double2 o = clf[ix];
+    o.x += f[k].x;
+    o.y += f[k].y;
+    clf[ix] = o;
+  }
+}
+
+// row i of the same, in d registers: the spinors come from L1
+template <int D>
+__device__ __forceinline__ void clover_slot_row(double2 *clf, const PoleSet &ps, const Geom &g, int id, int i, int slot) {
+  double2 f[D];
+  YG_UNROLL_DF
+  for (int j = 0; j < D; j++) f[j] = make_double2(0, 0);
+#pragma unroll 1
+  for (int n = 0; n < ps.n; n++) {
+    double2 l[4][1], r[4][1], sl[4][1], sr[4][1];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      l[k][0] = cscale(ps.lhs[n][fidx(g, id, k * D + i, 4 * D)], ps.w[n]);
+      r[k][0] = cscale(ps.rhs[n][fidx(g, id, k * D + i, 4 * D)], ps.w[n]);
+    }
+    g5_sigma<1>(sl, l, slot);
+    g5_sigma<1>(sr, r, slot);
+    YG_UNROLL_DF
+    for (int j = 0; j < D; j++) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        cfma(f[j], sl[k][0], cconj(ps.rhs[n][fidx(g, id, k * D + j, 4 * D)]));
+        cfma(f[j], sr[k][0], cconj(ps.lhs[n][fidx(g, id, k * D + j, 4 * D)]));
+      }
+    }
+  }
+  YG_UNROLL_DF
+  for (int j = 0; j < D; j++) {
+    const long ix = fidx(g, id, slot * D * D + i * D + j, 6 * D * D);
+    clf[ix] = cadd(clf[ix], f[j]);
+  }
+}
+
+// Which split: d <= 3 a warp per slot of 32 sites with a constant slot (sigma psi is a renaming of
+// psi's registers); d = 4 and d >= 8, where that spills, a warp per slot and row (blockIdx.y); d = 6
+// one thread a site, slot after slot and pole after pole (k_clover_fermion_site).  us for one pole, a
+// thread a site / this split: d = 3 32 x 16^3 134 / 118; d = 4 16^4 120 / 114; d = 8 12^4 720 / 124; d = 15
+// 8^4 1601 / 114 (d = 6 16^4: 286 a thread a site, 410 a row, 458 a slot).
+template <int D>
+__global__ void __launch_bounds__(192) k_clover_fermion_force(double2 *clf, const __grid_constant__ PoleSet ps, Geom g) {
+  const int id = blockIdx.x * 32 + (threadIdx.x & 31), i = blockIdx.y;
+  if (id >= g.V) return;
+  auto slot = [&](int sl) {
+    if (D <= 3) clover_slot_force<D>(clf, ps, g, id, sl);
+    else clover_slot_row<D>(clf, ps, g, id, i, sl);
+  };
+  switch (threadIdx.x >> 5) {
+    case 0: slot(0); break;
+    case 1: slot(1); break;
+    case 2: slot(2); break;
+    case 3: slot(3); break;
+    case 4: slot(4); break;
+    default: slot(5); break;
+  }
+}
+
+template <int D>
+__global__ void k_clover_fermion_site(double2 *clf, const double2 *lhs, const double2 *rhs, Geom g, double residue) {
   int id = blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= g.V) return;
   double2 l[4][D], r[4][D];
@@ -148,84 +329,152 @@ __global__ void k_clover_fermion_force(double2 *clf, const double2 *lhs, const d
   }
 }
 
-// ---- hopping force, forces.cpp:200-223 (all sites, all mu)
+// ---- hopping force, forces.cpp:200-223 (all sites, all mu), summed over the poles as above: a
+// warp takes one direction of 32 sites, accumulates sum_n c_n fmat_n, multiplies by U once and
+// projects once (the projection is linear, so the result equals the sum of the per-pole forces
+// up to rounding)
 template <int D>
-__global__ void k_hopping_force(double *mom, const double2 *lhs, const double2 *rhs, const double2 *U, Geom g,
-                                const double2 *itrepr, int ng, double coeff) {
-  long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (t >= 4L * g.V) return;
-  int id = (int)(t >> 2), mu = (int)(t & 3);
-  int c[4];
-  coords_of(g, id, c);
-  int fw = neighbour(g, c, mu, +1);
-  double2 a[4][D], b[4][D], tl[4][D], tr[4][D];
-  ld_spinor64<D>(a, lhs, g, fw);
-  g5_omg<D>(tl, a, mu);
-  ld_spinor64<D>(a, rhs, g, fw);
-  g5_omg<D>(tr, a, mu);
-  ld_spinor64<D>(a, rhs, g, id);
-  ld_spinor64<D>(b, lhs, g, id);
-  double2 f[D * D];
+__device__ __forceinline__ void hopping_fmat(double2 (&f)[D * D], const PoleSet &ps, const Geom &g, int id, int fw,
+                                             int mu) {
   YG_UNROLL_DF
   for (int k = 0; k < D * D; k++) f[k] = make_double2(0, 0);
-  outer_acc<D>(f, tl, a);
-  outer_acc<D>(f, tr, b);
-  double2 u[D * D], m[D * D];
-  ld_mat<D>(u, U, g, id, mu, 4);
-  mat_mul<D>(m, u, f);
-  project_add<D>(mom + (4L * id + mu) * ng, m, itrepr, ng, coeff);
-}
-
-// ---- _compute_clover_force, clover.cpp:170-262 (sites of block 1)
-template <int D>
-__global__ void k_clover_ldl_force(double2 *clf, const double2 *ldl, Geom g, double coeff) {
-  int h = blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= g.Vh) return;
-  int id = g.Vh + h;
-  constexpr int N = 2 * D, P = D * (2 * D + 1);
-  double2 A[2][N][N];
-  for (int blk = 0; blk < 2; blk++) {
-    const double2 *Lb = ldl + (long)blk * P * g.Vh + h;
-    for (int n = 0; n < N; n++) {
-      for (int i = 0; i < N; i++) A[blk][i][n] = make_double2(i == n ? coeff : 0.0, 0.0);
-      for (int i = n; i < N; i++)
-        for (int k = 0; k < i; k++)
-          A[blk][i][n] = csub(A[blk][i][n], cmul(Lb[(long)(i * (i + 1) / 2 + k) * g.Vh], A[blk][k][n]));
-      for (int i = N - 1; i >= n; i--) {
-        A[blk][i][n] = cscale(A[blk][i][n], 1.0 / Lb[(long)(i * (i + 1) / 2 + i) * g.Vh].x);
-        for (int k = i + 1; k < N; k++)
-          A[blk][i][n] = csub(A[blk][i][n], cmulc(Lb[(long)(k * (k + 1) / 2 + i) * g.Vh], A[blk][k][n]));
-      }
-    }
+#pragma unroll 1
+  for (int n = 0; n < ps.n; n++) {
+    double2 a[4][D], t[4][D];
+    ld_spinor64<D>(a, ps.lhs[n], g, fw);
+    g5_omg<D>(t, a, mu);
+    ld_spinor64<D>(a, ps.rhs[n], g, id);
+    scale_spinor<D>(a, ps.w[n]);
+    outer_acc<D>(f, t, a);
+    ld_spinor64<D>(a, ps.rhs[n], g, fw);
+    g5_omg<D>(t, a, mu);
+    ld_spinor64<D>(a, ps.lhs[n], g, id);
+    scale_spinor<D>(a, ps.w[n]);
+    outer_acc<D>(f, t, a);
   }
-  const double2(&a)[N][N] = A[0];
-  const double2(&b)[N][N] = A[1];
-  for (int i = 0; i < D; i++)
-    for (int j = 0; j < D; j++) {
-      double2 a21 = a[i + D][j], a12 = cconj(a[j + D][i]), a43 = b[i + D][j], a34 = cconj(b[j + D][i]);
-      double2 a11, a22, a33, a44;
-      if (i < j) {
-        a11 = cconj(a[j][i]); a22 = cconj(a[j + D][i + D]); a33 = cconj(b[j][i]); a44 = cconj(b[j + D][i + D]);
-      } else {
-        a11 = a[i][j]; a22 = a[i + D][j + D]; a33 = b[i][j]; a44 = b[i + D][j + D];
-      }
-      double2 F[6];
-      F[0] = make_double2(a12.y + a21.y - a34.y - a43.y, -a12.x - a21.x + a34.x + a43.x);   // X_01
-      F[1] = make_double2(a12.x - a21.x + a43.x - a34.x, a12.y - a21.y + a43.y - a34.y);    // X_02
-      F[2] = make_double2(a22.y - a11.y + a44.y - a33.y, a11.x - a22.x + a33.x - a44.x);    // X_12
-      F[3] = make_double2(a11.y - a22.y + a44.y - a33.y, a22.x - a11.x + a33.x - a44.x);    // X_03
-      F[4] = make_double2(a12.x - a21.x + a34.x - a43.x, a12.y - a21.y + a34.y - a43.y);    // X_13
-      F[5] = make_double2(-a12.y - a21.y - a34.y - a43.y, a12.x + a21.x + a34.x + a43.x);   // X_23
-      for (int s = 0; s < 6; s++) {
-        long ix = fidx(g, id, s * D * D + i * D + j, 6 * D * D);
-        clf[ix] = cadd(clf[ix], F[s]);
-      }
-    }
 }
 
-// ---- clover_force_core, forces.cpp:33-106
 template <int D>
-__global__ void k_clover_force_core(double *mom, const double2 *clf, const double2 *U, Geom g, const double2 *itrepr,
+__global__ void __launch_bounds__(128) k_hopping_force(double *mom, const __grid_constant__ PoleSet ps, const double2 *U,
+                                                       Geom g, const double2 *itrepr, int ng) {
+  extern __shared__ double mom_acc[];
+  const int site0 = blockIdx.x * 32, lane = threadIdx.x & 31, mu = threadIdx.x >> 5;
+  const int id = min(site0 + lane, g.V - 1);
+  int c[4];
+  coords_of(g, id, c);
+  const int fw = neighbour(g, c, mu, +1);
+  double2 f[D * D];
+  if (D > 6) hopping_fmat<D>(f, ps, g, id, fw, mu);
+  else if (mu == 0) hopping_fmat<D>(f, ps, g, id, fw, 0);
+  else if (mu == 1) hopping_fmat<D>(f, ps, g, id, fw, 1);
+  else if (mu == 2) hopping_fmat<D>(f, ps, g, id, fw, 2);
+  else hopping_fmat<D>(f, ps, g, id, fw, 3);
+  lmul<D, false>(f, U, g, id, mu, 4);
+  project_store<D, 33>(mom_acc + mu * ng * 33 + lane, f, itrepr, ng, 1.0);
+  add_momenta<4, 1>(mom, mom_acc, g, site0, 0, ng);
+}
+
+// ---- _compute_clover_force, clover.cpp:170-262 (sites of block 1): coeff times the entries of
+// A_oo^-1 combined into the six planes, from the packed Hermitian inverse the Schur operator
+// uses (layout of cpk_site).  Lane = site, one (i, j) colour pair per warp: each entry of the
+// inverse is read as it is needed and each word of cl_force updated once.
+template <int D>
+__device__ __forceinline__ double2 cpk_entry(const double2 *Cb, int Vh, int r, int c) {
+  if (r == c) {
+    const double2 d = __ldg(Cb + (long)(r >> 1) * Vh);
+    return make_double2((r & 1) ? d.y : d.x, 0.0);
+  }
+  const int hi = r > c ? r : c, lo = r > c ? c : r;
+  const double2 m = __ldg(Cb + (long)(D + hi * (hi - 1) / 2 + lo) * Vh);
+  return r > c ? m : cconj(m);
+}
+
+template <int D>
+__global__ void __launch_bounds__(256) k_clover_ldl_force(double2 *clf, const double2 *cpk, Geom g, double coeff) {
+  const int h = blockIdx.x * 32 + (threadIdx.x & 31);
+  const int ij = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (h >= g.Vh || ij >= D * D) return;
+  const int id = g.Vh + h, i = ij / D, j = ij % D;
+  const double2 *A = cpk + h, *B = A + 2L * D * D * g.Vh;
+  const double2 a21 = cscale(cpk_entry<D>(A, g.Vh, i + D, j), coeff), a12 = cscale(cpk_entry<D>(A, g.Vh, i, j + D), coeff);
+  const double2 a43 = cscale(cpk_entry<D>(B, g.Vh, i + D, j), coeff), a34 = cscale(cpk_entry<D>(B, g.Vh, i, j + D), coeff);
+  const double2 a11 = cscale(cpk_entry<D>(A, g.Vh, i, j), coeff), a22 = cscale(cpk_entry<D>(A, g.Vh, i + D, j + D), coeff);
+  const double2 a33 = cscale(cpk_entry<D>(B, g.Vh, i, j), coeff), a44 = cscale(cpk_entry<D>(B, g.Vh, i + D, j + D), coeff);
+  double2 F[6];
+  F[0] = make_double2(a12.y + a21.y - a34.y - a43.y, -a12.x - a21.x + a34.x + a43.x);   // X_01
+  F[1] = make_double2(a12.x - a21.x + a43.x - a34.x, a12.y - a21.y + a43.y - a34.y);    // X_02
+  F[2] = make_double2(a22.y - a11.y + a44.y - a33.y, a11.x - a22.x + a33.x - a44.x);    // X_12
+  F[3] = make_double2(a11.y - a22.y + a44.y - a33.y, a22.x - a11.x + a33.x - a44.x);    // X_03
+  F[4] = make_double2(a12.x - a21.x + a34.x - a43.x, a12.y - a21.y + a34.y - a43.y);    // X_13
+  F[5] = make_double2(-a12.y - a21.y - a34.y - a43.y, a12.x + a21.x + a34.x + a43.x);   // X_23
+#pragma unroll
+  for (int s = 0; s < 6; s++) {
+    const long ix = fidx(g, id, s * D * D + ij, 6 * D * D);
+    clf[ix] = cadd(clf[ix], F[s]);
+  }
+}
+
+// ---- clover_force_core, forces.cpp:33-106.  For each plane the eight terms of its two loops
+// through the link are, with A the side link at x (or its dagger), S the opposite link, C the far
+// side link and Z_a..Z_c the cl_force of the corners,
+//     C [ Z_s (S A) + S (Z_a A + A Z_0) ] + Z_1 (C S A),
+// up (A = U(x,nu)^dag, S = U(x+nu,mu)^dag, C = U(x+mu,nu)) minus down (A = U(x-nu,nu),
+// S = U(x-nu,mu)^dag, C = U(x-nu+mu,nu)^dag).  A block takes 32 sites and one direction mu, one
+// warp per nu != mu, and the projected planes are summed in shared memory.
+template <int D, bool UP>
+__device__ __forceinline__ void clover_loop(double2 (&t)[D * D], const double2 *clf, const double2 *U, const Geom &g,
+                                            int num, int mu, int nu, int x0, int x1, int aid, int sid, int cid, int za,
+                                            int zs) {
+  double2 p[D * D];
+  ld_mat<D>(t, clf, g, x0, num, 6);
+  lmul<D, UP>(t, U, g, aid, nu, 4);                       // A Z_0
+  ld_mat<D>(p, U, g, aid, nu, 4);
+  if (UP) {
+    double2 q[D * D];
+    dag<D>(q, p);
+    YG_UNROLL_DF
+    for (int k = 0; k < D * D; k++) p[k] = q[k];          // A
+  }
+  lmul_add<D>(t, p, clf, g, za, num, 6);                  // + Z_a A
+  lmul<D, true>(t, U, g, sid, mu, 4);                     // S (...)
+  lmul<D, true>(p, U, g, sid, mu, 4);                     // S A
+  lmul_add<D>(t, p, clf, g, zs, num, 6);                  // + Z_s (S A)
+  lmul<D, !UP>(t, U, g, cid, nu, 4);                      // C [...]
+  lmul<D, !UP>(p, U, g, cid, nu, 4);                      // C S A
+  lmul_add<D>(t, p, clf, g, x1, num, 6);                  // + Z_1 (C S A)
+}
+
+template <int D>
+__global__ void __launch_bounds__(96, (D <= 3 ? 4 : 2))
+    k_clover_force_core(double *mom, const double2 *clf, const double2 *U, Geom g, const double2 *itrepr, int ng,
+                        double coeff) {
+  extern __shared__ double mom_acc[];
+  const int site0 = (blockIdx.x >> 2) * 32, lane = threadIdx.x & 31, w = threadIdx.x >> 5, mu = blockIdx.x & 3;
+  const int id = min(site0 + lane, g.V - 1);
+  const int nu = w + (w >= mu);
+  int c[4], cc[4];
+  coords_of(g, id, c);
+  const int o1 = neighbour(g, c, mu, +1), o2 = neighbour(g, c, nu, +1), o3 = neighbour(g, c, nu, -1);
+  coords_of(g, o3, cc);
+  const int o4 = neighbour(g, cc, mu, +1);
+  coords_of(g, o2, cc);
+  const int o5 = neighbour(g, cc, mu, +1);
+  int num, sign;
+  if (mu < nu) { num = nu * (nu - 1) / 2 + mu; sign = 1; }
+  else { num = mu * (mu - 1) / 2 + nu; sign = -1; }
+  double2 F[D * D], t[D * D];
+  clover_loop<D, true>(F, clf, U, g, num, mu, nu, id, o1, id, o2, o1, o2, o5);
+  clover_loop<D, false>(t, clf, U, g, num, mu, nu, id, o1, o3, o3, o4, o3, o4);
+  YG_UNROLL_DF
+  for (int k = 0; k < D * D; k++) F[k] = csub(F[k], t[k]);
+  lmul<D, false>(F, U, g, id, mu, 4);
+  project_store<D, 33>(mom_acc + w * ng * 33 + lane, F, itrepr, ng, sign * coeff);
+  add_momenta<1, 3>(mom, mom_acc, g, site0, mu, ng);
+}
+
+// The same for larger d, one thread a link (the matrices live in local memory either way)
+template <int D>
+__global__ void k_clover_force_core_link(double *mom, const double2 *clf, const double2 *U, Geom g, const double2 *itrepr,
                                     int ng, double coeff) {
   long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (t >= 4L * g.V) return;
@@ -280,116 +529,36 @@ __global__ void k_clover_force_core(double *mom, const double2 *clf, const doubl
   }
 }
 
-// ---- the same two forces summed over the poles of a rational approximation
-// (rhmc.cpp:86-106 calls wilson_fermion_force_q once per pole): one thread per (site, slot)
-// accumulates sum_n w_n fmat_n in registers and updates cl_force once; one thread per
-// (site, mu) accumulates sum_n c_n fmat_n, multiplies by U once and projects once.  The
-// projection is linear, so the result equals the sum of the per-pole forces up to rounding.
-template <int D>
-__global__ void k_clover_fermion_force_multi(double2 *clf, PoleSet ps, Geom g) {
-  long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (t >= 6L * g.V) return;
-  const int id = (int)(t / 6), slot = (int)(t % 6);
-  double2 f[D * D];
-  YG_UNROLL_DF
-  for (int k = 0; k < D * D; k++) f[k] = make_double2(0, 0);
-#pragma unroll 1
-  for (int n = 0; n < ps.n; n++) {
-    double2 l[4][D], r[4][D], sl[4][D], sr[4][D], fn[D * D];
-    ld_spinor64<D>(l, ps.lhs[n], g, id);
-    ld_spinor64<D>(r, ps.rhs[n], g, id);
-    g5_sigma<D>(sl, l, slot);
-    g5_sigma<D>(sr, r, slot);
-    YG_UNROLL_DF
-    for (int k = 0; k < D * D; k++) fn[k] = make_double2(0, 0);
-    outer_acc<D>(fn, sl, r);
-    outer_acc<D>(fn, sr, l);
-    YG_UNROLL_DF
-    for (int k = 0; k < D * D; k++) {
-      f[k].x += ps.w[n] * fn[k].x;
-      f[k].y += ps.w[n] * fn[k].y;
-    }
-  }
-  YG_UNROLL_DF
-  for (int k = 0; k < D * D; k++) {
-    long ix = fidx(g, id, slot * D * D + k, 6 * D * D);
-    double2 o = clf[ix];
-    o.x += f[k].x;
-    o.y += f[k].y;
-    clf[ix] = o;
-  }
-}
-
-template <int D>
-__global__ void k_hopping_force_multi(double *mom, PoleSet ps, const double2 *U, Geom g, const double2 *itrepr,
-                                      int ng) {
-  long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (t >= 4L * g.V) return;
-  int id = (int)(t >> 2), mu = (int)(t & 3);
-  int c[4];
-  coords_of(g, id, c);
-  int fw = neighbour(g, c, mu, +1);
-  double2 f[D * D];
-  YG_UNROLL_DF
-  for (int k = 0; k < D * D; k++) f[k] = make_double2(0, 0);
-#pragma unroll 1
-  for (int n = 0; n < ps.n; n++) {
-    double2 a[4][D], b[4][D], tl[4][D], tr[4][D], fn[D * D];
-    ld_spinor64<D>(a, ps.lhs[n], g, fw);
-    g5_omg<D>(tl, a, mu);
-    ld_spinor64<D>(a, ps.rhs[n], g, fw);
-    g5_omg<D>(tr, a, mu);
-    ld_spinor64<D>(a, ps.rhs[n], g, id);
-    ld_spinor64<D>(b, ps.lhs[n], g, id);
-    YG_UNROLL_DF
-    for (int k = 0; k < D * D; k++) fn[k] = make_double2(0, 0);
-    outer_acc<D>(fn, tl, a);
-    outer_acc<D>(fn, tr, b);
-    YG_UNROLL_DF
-    for (int k = 0; k < D * D; k++) {
-      f[k].x += ps.w[n] * fn[k].x;
-      f[k].y += ps.w[n] * fn[k].y;
-    }
-  }
-  double2 u[D * D], m[D * D];
-  ld_mat<D>(u, U, g, id, mu, 4);
-  mat_mul<D>(m, u, f);
-  project_add<D>(mom + (4L * id + mu) * ng, m, itrepr, ng, 1.0);
-}
-
 // ------------------------------------------------------------------ launchers
 template <int D>
-void DK<D>::clover_fermion_force_multi(double2 *clf, const PoleSet &ps, Geom g, cudaStream_t s) {
-  k_clover_fermion_force_multi<D><<<nblk(6L * g.V, 64), 64, 0, s>>>(clf, ps, g);
+void DK<D>::clover_fermion_force(double2 *clf, const PoleSet &ps, Geom g, cudaStream_t s) {
+  if constexpr (D == 6) {
+    for (int n = 0; n < ps.n; n++)
+      k_clover_fermion_site<D><<<nblk(g.V, 64), 64, 0, s>>>(clf, ps.lhs[n], ps.rhs[n], g, ps.w[n]);
+  } else {
+    k_clover_fermion_force<D><<<dim3(nblk(g.V, 32), D <= 3 ? 1 : D), 192, 0, s>>>(clf, ps, g);
+  }
 }
 
 template <int D>
-void DK<D>::hopping_force_multi(double *mom, const PoleSet &ps, const double2 *U, Geom g, const double2 *itrepr,
-                                int ng, cudaStream_t s) {
-  k_hopping_force_multi<D><<<nblk(4L * g.V, 64), 64, 0, s>>>(mom, ps, U, g, itrepr, ng);
+void DK<D>::hopping_force(double *mom, const PoleSet &ps, const double2 *U, Geom g, const double2 *itrepr, int ng,
+                          cudaStream_t s) {
+  k_hopping_force<D><<<nblk(g.V, 32), 128, momenta_smem(4, ng), s>>>(mom, ps, U, g, itrepr, ng);
 }
 
 template <int D>
-void DK<D>::clover_fermion_force(double2 *clf, const double2 *lhs, const double2 *rhs, Geom g, double residue,
-                                 cudaStream_t s) {
-  k_clover_fermion_force<D><<<nblk(g.V, 64), 64, 0, s>>>(clf, lhs, rhs, g, residue);
-}
-
-template <int D>
-void DK<D>::hopping_force(double *mom, const double2 *lhs, const double2 *rhs, const double2 *U, Geom g,
-                          const double2 *itrepr, int ng, double coeff, cudaStream_t s) {
-  k_hopping_force<D><<<nblk(4L * g.V, 64), 64, 0, s>>>(mom, lhs, rhs, U, g, itrepr, ng, coeff);
-}
-
-template <int D>
-void DK<D>::clover_ldl_force(double2 *clf, const double2 *ldl, Geom g, double coeff, cudaStream_t s) {
-  k_clover_ldl_force<D><<<nblk(g.Vh, 64), 64, 0, s>>>(clf, ldl, g, coeff);
+void DK<D>::clover_ldl_force(double2 *clf, const double2 *cpk, Geom g, double coeff, cudaStream_t s) {
+  const int warps = D * D < 8 ? D * D : 8;
+  k_clover_ldl_force<D><<<dim3(nblk(g.Vh, 32), nblk(D * D, warps)), 32 * warps, 0, s>>>(clf, cpk, g, coeff);
 }
 
 template <int D>
 void DK<D>::clover_force_core(double *mom, const double2 *clf, const double2 *U, Geom g, const double2 *itrepr, int ng,
                               double coeff, cudaStream_t s) {
-  k_clover_force_core<D><<<nblk(4L * g.V, 64), 64, 0, s>>>(mom, clf, U, g, itrepr, ng, coeff);
+  if constexpr (D <= 6)
+    k_clover_force_core<D><<<4 * nblk(g.V, 32), 96, momenta_smem(3, ng), s>>>(mom, clf, U, g, itrepr, ng, coeff);
+  else
+    k_clover_force_core_link<D><<<nblk(4L * g.V, 64), 64, 0, s>>>(mom, clf, U, g, itrepr, ng, coeff);
 }
 
 }  // namespace yg

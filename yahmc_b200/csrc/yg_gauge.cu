@@ -98,115 +98,112 @@ __device__ __forceinline__ void add_scaled(double2 (&s)[N * N], const double2 (&
 }
 
 // ------------------------------------------------------------------ staples and forces
-// plaquette staples of link (x, mu): sum over nu of the two weighted 3-link paths
-template <int N>
-__device__ void staple_plaq(double2 (&st)[N * N], const double2 *U, const Geom &g, const Pos &x, int mu) {
-  double2 A[N * N], B[N * N], P[N * N], Q[N * N];
-#pragma unroll 1
-  for (int nu = 0; nu < 4; nu++) {
-    if (nu == mu) continue;
-    // U(x+mu, nu) [U(x, nu) U(x+nu, mu)]^dag
-    Pos o1 = step(g, x, mu, +1), o2 = step(g, x, nu, +1);
-    ldU<N>(A, U, g, x, nu); ldU<N>(B, U, g, o2, mu); mat_mul<N>(P, A, B);
-    ldU<N>(A, U, g, o1, nu); mul_dag<N>(Q, A, P);
-    add_scaled<N>(st, Q, plaq_w(g, x.c[0], mu, nu));
-    // [U(x-nu, mu) U(x-nu+mu, nu)]^dag U(x-nu, nu)
-    Pos b1 = step(g, x, nu, -1), b2 = step(g, b1, mu, +1);
-    ldU<N>(A, U, g, b1, mu); ldU<N>(B, U, g, b2, nu); mat_mul<N>(P, A, B);
-    ldU<N>(A, U, g, b1, nu); dag_mul<N>(Q, P, A);
-    add_scaled<N>(st, Q, plaq_w(g, b1.c[0], nu, mu));
+// Components of the algebra (suNa order, suNg.cpp:15-58) of c * Re tr(iT_a m) for the
+// fundamental generators, whose entries are 1, -1 and i off the diagonal: no table needed.
+// out[a * OST] for a = 0 .. N^2 - 2.
+template <int N, int OST>
+__device__ __forceinline__ void project_fund(double *out, const double2 (&m)[N * N], double c) {
+  int n = 0;
+#pragma unroll
+  for (int i = 0; i < N; i++)
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      if (i > j) {
+        out[(n++) * OST] = -c * (m[j * N + i].y + m[i * N + j].y);
+      } else if (i < j) {
+        out[(n++) * OST] = c * (m[j * N + i].x - m[i * N + j].x);
+      } else if (i > 0) {
+        double t = i * m[i * N + i].y;
+#pragma unroll
+        for (int k = 0; k < i; k++) t -= m[k * N + k].y;
+        out[(n++) * OST] = c * sqrt(2.0 / (i * (i + 1))) * t;
+      }
+    }
+}
+
+// X = the link (p, mu), or its dagger
+template <int N, bool DAG>
+__device__ __forceinline__ void ld_link(double2 (&X)[N * N], const double2 *U, const Geom &g, const Pos &p, int mu) {
+  double2 M[N * N];
+  ldU<N>(M, U, g, p, mu);
+#pragma unroll
+  for (int i = 0; i < N; i++)
+#pragma unroll
+    for (int j = 0; j < N; j++) X[i * N + j] = DAG ? cconj(M[j * N + i]) : M[i * N + j];
+}
+
+// Staples of link (x, mu) on one side of the plane (mu, nu): the plaquette C B^dag A with weight
+// c0 and, IMP = 1, its three 2x1 rectangles of staples_symanzik with weight c1, in which one of the
+// three links is replaced by its own staple away from the loop (primes):
+//     C [ B^dag (c0 A + c1 A') + c1 B' A ] + c1 C' (B^dag A).
+// UP: A = U(x,nu)^dag, B = U(x+nu,mu), C = U(x+mu,nu); else, from y = x-nu, A = U(y,nu),
+// B = U(y,mu), C = U(y+mu,nu)^dag.  Written as left multiplications of a running product: 11
+// matrix products a side, 14 path by path.
+template <int N, int IMP, bool UP>
+__device__ __forceinline__ void staple_side(double2 (&st)[N * N], const double2 *U, const Geom &g, const Pos &x, int mu,
+                                            int nu, double c0, double c1) {
+  const Pos y = UP ? x : step(g, x, nu, -1);                // the corner A starts from
+  const Pos b = UP ? step(g, x, nu, +1) : y;                // where B starts
+  const Pos xm = step(g, x, mu, +1), ym = UP ? xm : step(g, xm, nu, -1), bm = step(g, b, mu, +1);
+  double2 S[N * N], X[N * N];
+  ld_link<N, UP>(S, U, g, y, nu);
+  const double wp = c0 * (UP ? plaq_w(g, x.c[0], mu, nu) : plaq_w(g, y.c[0], nu, mu));
+#pragma unroll
+  for (int k = 0; k < N * N; k++) S[k] = make_double2(wp * S[k].x, wp * S[k].y);
+  if (IMP) {
+    // A' around x-mu: UP [U(x-mu+nu,mu)]^dag [U(x-mu,nu)]^dag U(x-mu,mu), else
+    // [U(z,mu)]^dag U(z,nu) U(x-mu,mu) with z = y-mu
+    const Pos xb = step(g, x, mu, -1), z = step(g, y, mu, -1), zb = step(g, b, mu, -1);
+    ld_link<N, false>(X, U, g, xb, mu);
+    lmul<N, UP>(X, U, g, z.id, nu, 4);
+    lmul<N, true>(X, U, g, zb.id, mu, 4);
+    add_scaled<N>(S, X, c1 * rect_w(g, z.c[0], nu, mu));
   }
-}
-
-// R = a (b c d)^dag e f  style products of the rectangle staples, with the three links
-// under the dagger multiplied first
-template <int N>
-__device__ __forceinline__ void prod3(double2 (&r)[N * N], const double2 *U, const Geom &g, const Pos &p0, int m0,
-                                      const Pos &p1, int m1, const Pos &p2, int m2) {
-  double2 A[N * N], B[N * N], C[N * N];
-  ldU<N>(A, U, g, p0, m0); ldU<N>(B, U, g, p1, m1); mat_mul<N>(C, A, B);
-  ldU<N>(A, U, g, p2, m2); mat_mul<N>(r, C, A);
-}
-
-// rectangle (2x1) staples of link (x, mu), staples_symanzik: for each nu the six paths
-// that close a 2x1 loop with the link
-template <int N>
-__device__ void staple_rect(double2 (&st)[N * N], const double2 *U, const Geom &g, const Pos &x, int mu) {
-  double2 H[N * N], D2[N * N], P[N * N], Q[N * N], A[N * N];
-#pragma unroll 1
-  for (int nu = 0; nu < 4; nu++) {
-    if (nu == mu) continue;
-    {  // U(x+mu,nu) U(x+mu+nu,nu) [U(x,nu) U(x+nu,nu) U(x+2nu,mu)]^dag
-      Pos o1 = step(g, x, mu, +1), o2 = step(g, o1, nu, +1), o3 = step(g, x, nu, +1), o4 = step(g, o3, nu, +1);
-      prod3<N>(H, U, g, x, nu, o3, nu, o4, mu);
-      ldU<N>(A, U, g, o1, nu); ldU<N>(D2, U, g, o2, nu); mat_mul<N>(P, A, D2);
-      mul_dag<N>(Q, P, H);
-      add_scaled<N>(st, Q, rect_w(g, x.c[0], mu, nu));
-    }
-    {  // [U(y,mu) U(y+mu,nu) U(y+mu+nu,nu)]^dag U(y,nu) U(y+nu,nu),  y = x-2nu
-      Pos o1 = step(g, x, nu, -1), o2 = step(g, o1, nu, -1), o3 = step(g, o2, mu, +1), o4 = step(g, o3, nu, +1);
-      prod3<N>(H, U, g, o2, mu, o3, nu, o4, nu);
-      ldU<N>(A, U, g, o2, nu); ldU<N>(D2, U, g, o1, nu); mat_mul<N>(P, A, D2);
-      dag_mul<N>(Q, H, P);
-      add_scaled<N>(st, Q, rect_w(g, o2.c[0], mu, nu));
-    }
-    {  // U(x+mu,mu) [U(y,mu) U(y+mu,mu) U(y+2mu,nu)]^dag U(y,nu),  y = x-nu
-      Pos o1 = step(g, x, nu, -1), o2 = step(g, o1, mu, +1), o3 = step(g, o2, mu, +1), o4 = step(g, x, mu, +1);
-      prod3<N>(H, U, g, o1, mu, o2, mu, o3, nu);
-      ldU<N>(A, U, g, o4, mu); mul_dag<N>(P, A, H);
-      ldU<N>(A, U, g, o1, nu); mat_mul<N>(Q, P, A);
-      add_scaled<N>(st, Q, rect_w(g, o1.c[0], nu, mu));
-    }
-    {  // U(x+mu,mu) U(x+2mu,nu) [U(x,nu) U(x+nu,mu) U(x+nu+mu,mu)]^dag
-      Pos o1 = step(g, x, mu, +1), o2 = step(g, o1, mu, +1), o3 = step(g, x, nu, +1), o4 = step(g, o3, mu, +1);
-      prod3<N>(H, U, g, x, nu, o3, mu, o4, mu);
-      ldU<N>(A, U, g, o1, mu); ldU<N>(D2, U, g, o2, nu); mat_mul<N>(P, A, D2);
-      mul_dag<N>(Q, P, H);
-      add_scaled<N>(st, Q, rect_w(g, x.c[0], nu, mu));
-    }
-    {  // [U(y,mu) U(y+mu,mu) U(y+2mu,nu)]^dag U(y,nu) U(y+nu,mu),  y = x-mu-nu
-      Pos o1 = step(g, x, mu, -1), o2 = step(g, o1, nu, -1), o3 = step(g, o2, mu, +1), o4 = step(g, o3, mu, +1);
-      prod3<N>(H, U, g, o2, mu, o3, mu, o4, nu);
-      ldU<N>(A, U, g, o2, nu); ldU<N>(D2, U, g, o1, mu); mat_mul<N>(P, A, D2);
-      dag_mul<N>(Q, H, P);
-      add_scaled<N>(st, Q, rect_w(g, o2.c[0], nu, mu));
-    }
-    {  // U(x+mu,nu) [U(y,nu) U(y+nu,mu) U(y+nu+mu,mu)]^dag U(y,mu),  y = x-mu
-      Pos o1 = step(g, x, mu, -1), o2 = step(g, o1, nu, +1), o3 = step(g, o2, mu, +1), o4 = step(g, x, mu, +1);
-      prod3<N>(H, U, g, o1, nu, o2, mu, o3, mu);
-      ldU<N>(A, U, g, o4, nu); mul_dag<N>(P, A, H);
-      ldU<N>(A, U, g, o1, mu); mat_mul<N>(Q, P, A);
-      add_scaled<N>(st, Q, rect_w(g, o1.c[0], nu, mu));
-    }
+  lmul<N, true>(S, U, g, b.id, mu, 4);                      // B^dag (...)
+  if (IMP) {
+    // B' A one step further along nu: UP U(x+mu+nu,nu) [U(x+2nu,mu)]^dag [U(x+nu,nu)]^dag A, else
+    // [U(y2+mu,nu)]^dag [U(y2,mu)]^dag U(y2,nu) A with y2 = y-nu
+    const Pos e = step(g, b, nu, UP ? +1 : -1), q = UP ? b : e, qm = step(g, q, mu, +1);
+    ld_link<N, UP>(X, U, g, y, nu);
+    lmul<N, UP>(X, U, g, q.id, nu, 4);
+    lmul<N, true>(X, U, g, e.id, mu, 4);
+    lmul<N, !UP>(X, U, g, qm.id, nu, 4);
+    add_scaled<N>(S, X, c1 * rect_w(g, UP ? x.c[0] : e.c[0], mu, nu));
+  }
+  lmul<N, !UP>(S, U, g, ym.id, nu, 4);                      // C [...]
+  add_scaled<N>(st, S, 1.0);
+  if (IMP) {
+    // C' B^dag A around x+mu: UP U(x+mu,mu) U(x+2mu,nu) [U(x+mu+nu,mu)]^dag B^dag A, else
+    // U(x+mu,mu) [U(y+2mu,nu)]^dag [U(y+mu,mu)]^dag B^dag A
+    ld_link<N, UP>(X, U, g, y, nu);
+    lmul<N, true>(X, U, g, b.id, mu, 4);
+    lmul<N, true>(X, U, g, bm.id, mu, 4);
+    lmul<N, !UP>(X, U, g, step(g, ym, mu, +1).id, nu, 4);
+    lmul<N, false>(X, U, g, xm.id, mu, 4);
+    add_scaled<N>(st, X, c1 * rect_w(g, y.c[0], nu, mu));
   }
 }
 
 // mom(x,mu) -= algebra_project(U(x,mu) (c0 S_plaq + c1 S_rect), coeff); IMP = 0 skips the
-// rectangles (wilson_gauge_force, c0 = 1)
+// rectangles (wilson_gauge_force, c0 = 1).  A block takes 32 sites and one direction, one warp
+// per plane: every link load of a warp is a contiguous run, three threads share a link's chain
+// of products, and their algebra components meet in shared memory.
 template <int N, int IMP>
-__global__ void __launch_bounds__(64) k_gauge_force(double *mom, const double2 *U, Geom g, const double2 *itfund,
-                                                    double coeff, double c0, double c1) {
-  long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (t >= 4L * g.V) return;
-  const int id = (int)(t >> 2), mu = (int)(t & 3);
-  const Pos x = pos_of(g, id);
-  double2 sw[N * N], F[N * N], A[N * N];
+__global__ void __launch_bounds__(96, (N <= 3 ? 4 : 2))
+    k_gauge_force(double *mom, const double2 *U, Geom g, double coeff, double c0, double c1) {
+  constexpr int NG = N * N - 1;
+  __shared__ double acc[3 * NG * 33];
+  const int site0 = (blockIdx.x >> 2) * 32, lane = threadIdx.x & 31, w = threadIdx.x >> 5, mu = blockIdx.x & 3;
+  const int nu = w + (w >= mu);
+  const Pos x = pos_of(g, min(site0 + lane, g.V - 1));
+  double2 st[N * N];
 #pragma unroll
-  for (int k = 0; k < N * N; k++) sw[k] = make_double2(0, 0);
-  staple_plaq<N>(sw, U, g, x, mu);
-  if (IMP) {
-    double2 sr[N * N];
-#pragma unroll
-    for (int k = 0; k < N * N; k++) {
-      sr[k] = make_double2(0, 0);
-      sw[k] = make_double2(c0 * sw[k].x, c0 * sw[k].y);
-    }
-    staple_rect<N>(sr, U, g, x, mu);
-    add_scaled<N>(sw, sr, c1);
-  }
-  ldU<N>(A, U, g, x, mu);
-  mat_mul<N>(F, A, sw);
-  project_add<N>(mom + (4L * id + mu) * (N * N - 1), F, itfund, N * N - 1, -coeff);
+  for (int k = 0; k < N * N; k++) st[k] = make_double2(0, 0);
+  staple_side<N, IMP, true>(st, U, g, x, mu, nu, c0, c1);
+  staple_side<N, IMP, false>(st, U, g, x, mu, nu, c0, c1);
+  lmul<N, false>(st, U, g, x.id, mu, 4);
+  project_fund<N, 33>(acc + w * NG * 33 + lane, st, 0.5 * coeff);     // -coeff / -TF
+  add_momenta<1, 3>(mom, acc, g, site0, mu, NG);
 }
 
 // ------------------------------------------------------------------ Wilson loops
@@ -552,13 +549,11 @@ __global__ void k_mom_gaussian(double *mom, long nlinks, int ng, unsigned long l
 // ------------------------------------------------------------------ host side
 template <int N>
 static void launch_gauge_force(Lattice &L, double coeff, double c0, double c1, bool improved) {
-  const long n = 4L * L.V;
+  const int n = 4 * nblk(L.V, 32);
   if (improved)
-    k_gauge_force<N, 1><<<nblk(n, 64), 64, 0, L.stream>>>(L.mom.as<double>(), L.fund.as<double2>(), L.g, L.rt.itfund,
-                                                           coeff, c0, c1);
+    k_gauge_force<N, 1><<<n, 96, 0, L.stream>>>(L.mom.as<double>(), L.fund.as<double2>(), L.g, coeff, c0, c1);
   else
-    k_gauge_force<N, 0><<<nblk(n, 64), 64, 0, L.stream>>>(L.mom.as<double>(), L.fund.as<double2>(), L.g, L.rt.itfund,
-                                                           coeff, 1.0, 0.0);
+    k_gauge_force<N, 0><<<n, 96, 0, L.stream>>>(L.mom.as<double>(), L.fund.as<double2>(), L.g, coeff, 1.0, 0.0);
   YG_LAUNCHED();
 }
 

@@ -7,8 +7,7 @@ template void DK<10>::hop(const HopArgs<double> &, int, cudaStream_t);
 template void DK<10>::hop(const HopArgs<float> &, int, cudaStream_t);
 template void DK<10>::clover(double2 *, const double2 *, const double2 *, Geom, double, double, int, int, int, cudaStream_t);
 template void DK<10>::clover_inv(double2 *, const double2 *, const double2 *, Geom, int, cudaStream_t);
-template void DK<10>::ldl(double2 *, const double2 *, Geom, double, double, int, cudaStream_t);
+template void DK<10>::ldl_inverse(double2 *, double2 *, const double2 *, Geom, double, double, int, cudaStream_t);
 template void DK<10>::cinv_float(float2 *, const double2 *, int, cudaStream_t);
-template void DK<10>::cinv_packed64(double2 *, const double2 *, int, cudaStream_t);
 template void DK<10>::logdet(double *, const double2 *, int, cudaStream_t);
 }  // namespace yg

@@ -7,8 +7,7 @@ template void DK<15>::hop(const HopArgs<double> &, int, cudaStream_t);
 template void DK<15>::hop(const HopArgs<float> &, int, cudaStream_t);
 template void DK<15>::clover(double2 *, const double2 *, const double2 *, Geom, double, double, int, int, int, cudaStream_t);
 template void DK<15>::clover_inv(double2 *, const double2 *, const double2 *, Geom, int, cudaStream_t);
-template void DK<15>::ldl(double2 *, const double2 *, Geom, double, double, int, cudaStream_t);
+template void DK<15>::ldl_inverse(double2 *, double2 *, const double2 *, Geom, double, double, int, cudaStream_t);
 template void DK<15>::cinv_float(float2 *, const double2 *, int, cudaStream_t);
-template void DK<15>::cinv_packed64(double2 *, const double2 *, int, cudaStream_t);
 template void DK<15>::logdet(double *, const double2 *, int, cudaStream_t);
 }  // namespace yg

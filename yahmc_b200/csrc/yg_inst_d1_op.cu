@@ -7,8 +7,7 @@ template void DK<1>::hop(const HopArgs<double> &, int, cudaStream_t);
 template void DK<1>::hop(const HopArgs<float> &, int, cudaStream_t);
 template void DK<1>::clover(double2 *, const double2 *, const double2 *, Geom, double, double, int, int, int, cudaStream_t);
 template void DK<1>::clover_inv(double2 *, const double2 *, const double2 *, Geom, int, cudaStream_t);
-template void DK<1>::ldl(double2 *, const double2 *, Geom, double, double, int, cudaStream_t);
+template void DK<1>::ldl_inverse(double2 *, double2 *, const double2 *, Geom, double, double, int, cudaStream_t);
 template void DK<1>::cinv_float(float2 *, const double2 *, int, cudaStream_t);
-template void DK<1>::cinv_packed64(double2 *, const double2 *, int, cudaStream_t);
 template void DK<1>::logdet(double *, const double2 *, int, cudaStream_t);
 }  // namespace yg

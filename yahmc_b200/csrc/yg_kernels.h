@@ -9,8 +9,7 @@
 
 namespace yg {
 
-// CLOVINV applies the LDL factors (FP64) or the explicit inverse (FP32); CLOVPK the packed
-// Hermitian FP64 inverse
+// CLOVINV applies the explicit FP32 inverse, CLOVPK the packed Hermitian FP64 inverse
 enum { EPI_PLAIN = 0, EPI_CLOVINV = 1, EPI_CLOVADD = 2, EPI_AXPY = 3, EPI_CLOVPK = 4 };
 
 template <typename R>
@@ -22,9 +21,8 @@ struct HopArgs {
   cplx<R> *dst2;          // CLOVINV: also store the raw hop here (the reference's in-place write)
   const cplx<R> *src2;    // CLOVADD / AXPY: psi at the output site
   const cplx<R> *cl;      // clover term (4 d x d per site)
-  const double2 *ldl;     // LDL factors (FP64 path)
   const cplx<R> *cinv;    // explicit inverse clover blocks (FP32 path): 2 x (2d)^2 per site
-  const double2 *cpk;     // packed Hermitian inverse clover blocks (FP64 path, d <= 6): 2 x 2d^2 words per site
+  const double2 *cpk;     // packed Hermitian inverse clover blocks (FP64 path): 2 x 2d^2 words per site
   R coeff;                // -sign/2
   R diag;                 // 4+m (CLOVADD) or the AXPY coefficient
   R cfm1;                 // cf-1 (Dirac boundary term at t = Ta, Tb)
@@ -34,7 +32,7 @@ struct HopArgs {
   int zero_add_at_boundary;
 };
 
-// The fields of several pseudo-fermion poles for one batched force launch
+// The fields of the pseudo-fermion poles of one force launch (one for the plain force)
 constexpr int kMaxPoles = 32;
 struct PoleSet {
   const double2 *lhs[kMaxPoles];
@@ -51,19 +49,16 @@ struct DK {
   static void clover(double2 *dst, const double2 *src, const double2 *cl, Geom g, double mass4, double cfm1, int lo,
                      int n, int assign, cudaStream_t s);
   static void clover_inv(double2 *dst, const double2 *src, const double2 *ldl, Geom g, int assign, cudaStream_t s);
-  static void ldl(double2 *ldl, const double2 *cl, Geom g, double sigma, double cf, int boundary_term, cudaStream_t s);
+  // the LDL factors of A_oo and its packed Hermitian inverse
+  static void ldl_inverse(double2 *ldl, double2 *cpk, const double2 *cl, Geom g, double sigma, double cf,
+                          int boundary_term, cudaStream_t s);
   static void cinv_float(float2 *cinv, const double2 *ldl, int Vh, cudaStream_t s);
-  static void cinv_packed64(double2 *cpk, const double2 *ldl, int Vh, cudaStream_t s);
   static void logdet(double *out, const double2 *ldl, int Vh, cudaStream_t s);
-  static void clover_fermion_force(double2 *clf, const double2 *lhs, const double2 *rhs, Geom g, double residue,
-                                   cudaStream_t s);
-  static void hopping_force(double *mom, const double2 *lhs, const double2 *rhs, const double2 *U, Geom g,
-                            const double2 *itrepr, int ng, double coeff, cudaStream_t s);
-  static void clover_ldl_force(double2 *clf, const double2 *ldl, Geom g, double coeff, cudaStream_t s);
   // sums over the poles of a PoleSet, one read-modify-write of cl_force / the momenta
-  static void clover_fermion_force_multi(double2 *clf, const PoleSet &ps, Geom g, cudaStream_t s);
-  static void hopping_force_multi(double *mom, const PoleSet &ps, const double2 *U, Geom g, const double2 *itrepr,
-                                  int ng, cudaStream_t s);
+  static void clover_fermion_force(double2 *clf, const PoleSet &ps, Geom g, cudaStream_t s);
+  static void hopping_force(double *mom, const PoleSet &ps, const double2 *U, Geom g, const double2 *itrepr, int ng,
+                            cudaStream_t s);
+  static void clover_ldl_force(double2 *clf, const double2 *cpk, Geom g, double coeff, cudaStream_t s);
   static void clover_force_core(double *mom, const double2 *clf, const double2 *U, Geom g, const double2 *itrepr,
                                 int ng, double coeff, cudaStream_t s);
 };

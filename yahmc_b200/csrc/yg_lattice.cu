@@ -252,15 +252,12 @@ void ensure_ldl(Lattice &L, double sigma) {
   if (!L.p.clover) return;
   if (L.ldl_valid && L.ldl_sigma == sigma) return;    // clover.cpp:314-321
   int boundary_term = (L.p.bc == YG_BC_OPEN || L.p.bc == YG_BC_SF);
-  YG_DISPATCH_D(L.d, K::ldl(L.ldl.as<double2>(), L.clover.as<double2>(), L.g, sigma, L.p.cf, boundary_term, L.stream));
+  // the Schur step of the FP64 operator and the clover force use the explicit inverse (a Hermitian
+  // mat-vec instead of the LDL substitutions): same matrix, no serial divide chain
+  L.cpk64.alloc(sizeof(double2) * 2 * 2 * (size_t)L.d * L.d * L.Vh);
+  YG_DISPATCH_D(L.d, K::ldl_inverse(L.ldl.as<double2>(), L.cpk64.as<double2>(), L.clover.as<double2>(), L.g, sigma,
+                                    L.p.cf, boundary_term, L.stream));
   YG_LAUNCHED();
-  if (L.d <= kPackedInverseMaxD) {
-    // the Schur step of the FP64 operator applies this explicit inverse (a Hermitian
-    // mat-vec) instead of the LDL substitutions: same matrix, no serial divide chain
-    L.cpk64.alloc(sizeof(double2) * 2 * 2 * (size_t)L.d * L.d * L.Vh);
-    YG_DISPATCH_D(L.d, K::cinv_packed64(L.cpk64.as<double2>(), L.ldl.as<double2>(), (int)L.Vh, L.stream));
-    YG_LAUNCHED();
-  }
   L.ldl_sigma = sigma;
   L.ldl_valid = true;
 }

@@ -65,7 +65,7 @@ struct Lattice {
   DevBuf ldl;       // LDL factors, 2 x d(2d+1) per site of block 1   (cl_ldl)
   double ldl_sigma = 0;
   bool ldl_valid = false;
-  DevBuf cpk64;     // packed Hermitian FP64 inverse of the odd-site blocks, d <= 6 (rebuilt with ldl)
+  DevBuf cpk64;     // packed Hermitian FP64 inverse of the odd-site blocks (rebuilt with ldl)
   DevBuf cl_force;  // 6 x d x d per site                            (cl_force)
   DevBuf mom;       // 4 x NG per site                               (afield_momenta)
   DevBuf tables;    // basis / generators
@@ -134,7 +134,6 @@ struct Lattice {
 Lattice *lattice_create(const yg_params &p);
 void represent_and_clover(Lattice &L);
 void ensure_ldl(Lattice &L, double sigma);
-constexpr int kPackedInverseMaxD = 6;   // largest d whose FP64 Schur step uses the packed inverse
 void gauge_upload(Lattice &L, const double *host);
 void gauge_upload_fund(Lattice &L, const double *host);
 void gauge_download(Lattice &L, double *host);
