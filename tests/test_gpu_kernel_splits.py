@@ -1,0 +1,85 @@
+"""The work splits of the FP64 kernels where they change over or leave remainders: four lanes a site up
+to kQuadSites = 4736 output sites and one thread a site above (d <= 6), blocks of 32 sites of the force
+and clover kernels with a ragged last block, and both splits of the persistent CG.  Against the FP64
+oracle; 1e-13 relative as in the parity tests of these functions (sums of a few hundred terms of
+relative rounding 1.1e-16)."""
+import numpy as np
+import pytest
+
+from tests.helpers import make_pair, rel, source
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-13
+ABOVE = (8, 10, 10, 12)          # 4800 even sites: one thread a site, a ragged last block of 128
+BELOW = (2, 6, 6, 6)             # 216 even sites: four lanes a site, 13.5 blocks of 32 sites
+
+
+@pytest.mark.parametrize("dims", [ABOVE, BELOW])
+@pytest.mark.parametrize("name", ["su3_fund_ap", "su2_adj_ap", "su4_fund_ap", "su3_sym_ap", "su3_fund_open",
+                                  "su3_fund_ap_nocl", "su3_fund_ap_full"])
+def test_operator(name, dims):
+    if name == "su3_fund_open" and dims[0] < 4:
+        dims = (4, 6, 6, 6)
+    lat, O, rng = make_pair(name, dims, seed=21)
+    src = source(O, rng)
+    for fn, args in (("Dphi", [-0.6]), ("Hphi_sq", [-0.4])):
+        s, d = lat.field(src), lat.field()
+        s2, d2 = src.copy(), O.new_field()
+        getattr(lat, fn)(*args, d, s)
+        getattr(O, fn)(*args, d2, s2)
+        assert rel(lat.download(d), d2) < TOL
+        assert rel(lat.download(s), s2) < TOL
+    if O.p.clover and O.p.eo:
+        lo = O.compute_ldl(4 - 0.4)
+        assert rel(lat.ldl(-0.4)[O.Vh:], lo[O.Vh:]) < TOL
+
+
+@pytest.mark.parametrize("name", ["su3_fund_ap", "su2_adj_ap", "su4_fund_ap", "su3_sym_ap", "su3_adj_ap", "su3_fund_sf"])
+def test_forces_ragged(name):
+    dims = (6, 2, 6, 6) if name.endswith("sf") else BELOW
+    lat, O, rng = make_pair(name, dims, seed=22)
+    a0, b0 = source(O, rng), source(O, rng)
+    a, b = lat.field(a0), lat.field(b0)
+    lat.zero_momenta()
+    O.mom[:] = 0
+    lat.begin_fermion_force()
+    O.begin_fermion_force()
+    lat.wilson_fermion_force_q_multi(0.1, -0.5, [0.7, -0.2], [a, b])
+    for f, w in ((a0, 0.7), (b0, -0.2)):
+        O.wilson_fermion_force_q(0.1, -0.5, w, f.copy())
+    lat.clover_logdet_force(-0.5, 2.0)
+    O.clover_logdet_force(-0.5, 2.0)
+    assert rel(lat.clover_force(), O.cl_force, floor=1.0) < TOL
+    lat.end_fermion_force(0.1)
+    O.end_fermion_force(0.1)
+    lat.improved_gauge_force(0.1, 5.6, 5.0 / 3.0, -1.0 / 12.0)
+    O.improved_gauge_force(0.1, 5.6, 5.0 / 3.0, -1.0 / 12.0)
+    lat.wilson_gauge_force(0.05, 5.6)
+    O.wilson_gauge_force(0.05, 5.6)
+    assert rel(lat.momenta(), O.mom, floor=1.0) < TOL
+    assert rel(lat.clover_term(), O.cl_term, floor=1.0) < TOL
+
+
+@pytest.mark.parametrize("name,dims", [("su3_fund_ap", ABOVE), ("su3_fund_ap", BELOW), ("su3_fund_ap_nocl", BELOW),
+                                       ("su3_sym_ap", BELOW), ("su2_fund_ap", (4, 4, 4, 6))])
+def test_persistent_cg(name, dims):
+    """One lattice per call of cg_inverter: the true residual meets prec and the solution is the
+    oracle's CG's (both solve to 1e-11 of |b|; the operator's condition number here is below 1e4)."""
+    lat, O, rng = make_pair(name, dims, seed=23)
+    b0 = source(O, rng)
+    b, x = lat.field(b0), lat.field()
+    it = lat.cg_inverter("Hphi_sq", 0.2, 1e-22, x, b)
+    xo = O.new_field()
+    ito = O.cg("Hphi_sq", 0.2, 1e-22, xo, b0.copy())
+    ito = ito[0] if isinstance(ito, tuple) else ito
+    assert abs(it - ito) <= 1
+    assert rel(lat.download(x)[:O.Vh], xo[:O.Vh]) < 1e-7
+    q = O.new_field()
+    xs = lat.download(x)
+    O.Hphi_sq(0.2, q, xs)
+    r = (q - b0)[:O.Vh]
+    assert np.vdot(r, r).real < 4e-22 * np.vdot(b0[:O.Vh], b0[:O.Vh]).real
+    # a call that starts from the solution makes no iteration, and maxiter ends a solve early
+    assert lat.cg_inverter("Hphi_sq", 0.2, 1e-20, x, b) == 0
+    lat.spinor_zero(x)
+    assert lat.cg_inverter("Hphi_sq", 0.2, 1e-22, x, b, maxiter=3) == 3 and lat.last_status == 4

@@ -9,28 +9,33 @@
 // CG loop on the device:
 //
 //   P1  o = A_oo^-1 (1/2 H p)              (odd sites)
-//   P2  t = g5 (A_ee p - 1/2 H o)          (even sites)          t = Hphi p
+//   P2  t = g5 (A_ee p - 1/2 H o), |t|^2   (even sites)          t = Hphi p
 //   P3  o = A_oo^-1 (1/2 H t)
-//   P4  q = g5 (A_ee t - 1/2 H o), <p,q>   (even sites)          q = Hphi_sq p
-//   P5  x += alpha p, r -= alpha q, |r|^2
-//   P6  p = beta p + r
+//   P4  q = g5 (A_ee t - 1/2 H o)          (even sites)          q = Hphi_sq p, never stored:
+//       r -= alpha q, |r|^2
+//   P5  x += alpha p, p = beta p + r
 //
-// with a barrier of the group after each phase.  The operator steps are the FP64 Schur steps
-// of the single-lattice path (hop_body of yg_dirac_impl.cuh with the same epilogues), and the
-// scalars are the reference's: alpha = rr / <p,q>, beta = rr_new / rr, stop when
+// with a barrier of the group after each phase.  Hphi is Hermitian on these lattices (no open or
+// SF slices), so <p, Hphi_sq p> = |Hphi p|^2 and alpha is known before the second Hphi ends, which
+// leaves five barriers an iteration and no pass over q.  The operator steps are the FP64 Schur
+// steps of the single-lattice path (yg_dirac_impl.cuh: four lanes a site up to kQuadSites) with ordinary loads for the
+// fields, which the kernel also writes.  The scalars are the reference's: alpha = rr / <p,q>, beta = rr_new / rr, stop when
 // rr_new < prec |b|^2, iteration count as cg_inverter's.  Reductions are deterministic: one
 // partial per block, which every block of the group adds in block order after the barrier,
 // so all blocks of a group hold the same alpha and beta.  Groups never wait for each other:
 // a lattice that converges early just ends its blocks.
 //
-// Barriers: a counter and a generation word per group in global memory.  Every wait is
-// bounded by a cycle limit; a block whose wait runs out sets the launch's error flag and
-// returns, every other block returns at its next barrier once the flag is set, and the host
-// reports YG_TIMEOUT.  The launch is cooperative, so all blocks are resident and in a healthy
-// run every barrier completes; the limit is the guard against anything else.
+// Barriers: one arrival counter per group, on a line of its own, that only grows; a block
+// releases its writes with its arrival and acquires the others' by polling the counter up to the
+// group's next multiple, one round trip each.  Every wait is bounded by a cycle limit; a block whose
+// wait runs out sets the launch's error flag and returns, every other block meets the flag in its
+// next wait (the missing arrival keeps it there) and returns too, and the host reports YG_TIMEOUT.
+// The launch is cooperative, so all blocks are resident and in a healthy run every barrier
+// completes; the limit is the guard against anything else.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <mutex>
 #include <vector>
 #include "yg_lattice.h"
 #include "yg_kernels.h"
@@ -40,15 +45,33 @@ namespace yg {
 
 namespace {
 
+// Two persistent grids at once could each hold multiprocessors that the other one's blocks need: one
+// runs at a time in a process.
+std::mutex g_persistent;
+
 constexpr int kThreads = 128;
+constexpr int kSyncStride = 32;                     // words between the groups' counters: 128 bytes
+
 constexpr long long kDefaultWait = 20000000000LL;   // cycles (about 10 s at 2 GHz)
 
+constexpr int kMaxLattices = 64;
+constexpr int kSiteMaxD = 4;                        // d = 6 with a thread a site spills under 168 registers
+
 struct BLat {
-  HopArgs<double> s1a, s2a, s1b, s2b;   // P1, P2, P3, P4
-  double2 *x, *r, *p, *q;              // even-site words of the whole-field layout
+  Geom g;
+  const double2 *U, *cl, *cpk;
+  double2 *x, *r, *p, *t, *o;          // whole-field layout; x, r, p, t even sites, o odd
   int b0, nb;                          // the group's blocks [b0, b0 + nb)
+  int quad;                            // four lanes a site instead of one thread
   int maxiter, it0;                    // it0 = -1: solved by the initial guess, no iteration
-  double target, rr0;                  // prec |b|^2, |r|^2 of the initial residual
+  double diag, target, rr0;            // diagonal of A_ee, prec |b|^2, |r|^2 of the initial residual
+};
+
+// A kernel parameter: geometry and pointers stay in the constant bank.  Read from global memory they
+// are loaded again after every store, which doubled the time of a step on 16^4.
+struct BArgs {
+  BLat l[kMaxLattices];
+  int n;
 };
 
 struct BOut {
@@ -76,137 +99,168 @@ __device__ __forceinline__ double group_total(const double *part, int b0, int nb
   return block_sum(acc);
 }
 
-// barrier of the nb blocks of a group; false when this block's wait ran out or another
-// block of the launch gave up (the error flag is set), in which case the block returns
-__device__ __forceinline__ bool group_sync(unsigned *cnt, unsigned *gen, unsigned nb, int *err, long long limit) {
+// barrier of the nb blocks of a group: `due` counts the arrivals of all barriers so far.  False
+// when this block's wait ran out or another block of the launch gave up: the block returns.
+__device__ __forceinline__ bool group_sync(unsigned *cnt, unsigned &due, unsigned nb, int *err, long long limit) {
   __shared__ int ok;
+  due += nb;
   __syncthreads();
   if (threadIdx.x == 0) {
     int good = 1;
-    volatile unsigned *vgen = gen;
-    volatile int *verr = err;
-    const unsigned g0 = *vgen;
-    __threadfence();                                   // this block's stores before its arrival
-    if (atomicAdd(cnt, 1u) == nb - 1) {
-      atomicExch(cnt, 0u);
-      __threadfence();
-      atomicAdd(gen, 1u);
-    } else {
-      const long long t0 = clock64();
-      while (*vgen == g0) {
-        if (*verr) { good = 0; break; }
-        if (clock64() - t0 > limit) { atomicExch(err, 1); good = 0; break; }
-        __nanosleep(100);
-      }
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
+    const long long t0 = clock64();
+    while (true) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
+      if ((int)(v - due) >= 0) break;
+      if (*reinterpret_cast<volatile int *>(err)) { good = 0; break; }
+      if (clock64() - t0 > limit) { atomicExch(err, 1); good = 0; break; }
     }
-    __threadfence();
-    if (*verr) good = 0;
     ok = good;
   }
   __syncthreads();
   return ok != 0;
 }
 
-// the two Schur steps as called functions, one body each however often the loop calls them
-template <int D, int EPI>
-__device__ __noinline__ void step(const HopArgs<double> &a, int t) {
-  hop_body<D, double, EPI>(a, t);
+// One word of a Schur step's result: stored as t (second = false) with its square, or taken as q,
+// r -= alpha q, with the square of the new r.
+__device__ __forceinline__ double finish(double2 v, bool second, double2 *t, double2 *r, double alpha, long i) {
+  if (!second) {
+    t[i] = v;
+  } else {
+    const double2 rv = r[i];
+    v = make_double2(fma(-alpha, v.x, rv.x), fma(-alpha, v.y, rv.y));
+    r[i] = v;
+  }
+  return fma(v.x, v.x, v.y * v.y);
+}
+
+// The whole CG loop of one lattice's group.  QUAD: four lanes a site (dead lanes, beyond the lattice,
+// take part), else a site per thread.  Both Hphi of an iteration run through the same two step bodies.
+template <int D, int CLOV, bool QUAD>
+__device__ __forceinline__ void group_cg(const BLat &L, double *part_pq, double *part_rr, unsigned *cnt, int *err,
+                                         BOut *out, long long limit) {
+  constexpr int E1 = CLOV ? EPI_CLOVPK : EPI_PLAIN, E2 = CLOV ? EPI_CLOVADD : EPI_AXPY;
+  constexpr int kSites = QUAD ? kThreads / 4 : kThreads;              // sites per block and pass
+  const int lb = blockIdx.x - L.b0, nb = L.nb, Vh = L.g.Vh;
+  const int stride = nb * kSites, passes = (Vh + stride - 1) / stride;
+  const int first = lb * kSites + (QUAD ? threadIdx.x >> 2 : threadIdx.x);
+  HopArgs<double> a{}, e{};
+  a.g = L.g; a.U = L.U; a.cpk = L.cpk; a.dst = L.o; a.lo = Vh; a.n = Vh; a.coeff = 0.5;
+  e.g = L.g; e.U = L.U; e.cl = L.cl; e.src = L.o; e.lo = 0; e.n = Vh; e.coeff = -0.5; e.diag = L.diag; e.g5 = 1;
+  e.zero_add_at_boundary = 1;
+  unsigned due = 0;
+  double rr = L.rr0, alpha = 0.0;
+  int it = 0, status = YG_OK;
+  // cg.cpp:151-153: a system solved by its initial guess returns 0 iterations
+  while (L.it0 == 0 && status == YG_OK) {
+    ++it;
+    if (L.maxiter > 0 && it > L.maxiter) { it--; status = YG_MAXITER; break; }
+#pragma unroll 1
+    for (int half = 0; half < 2; half++) {
+      a.src = half ? L.t : L.p;
+      e.src2 = a.src;
+      for (int k = 0; k < passes; k++) {
+        const int t = first + k * stride;
+        const bool live = t < Vh;
+        if (QUAD) {
+          double2 w[D];
+          long at;
+          hop_quad<D, double, E1, false>(a, live ? t : Vh - 1, live, w, at);
+          if (live) {
+#pragma unroll
+            for (int c = 0; c < D; c++) L.o[at + (long)c * Vh] = w[c];
+          }
+        } else if (live) {
+          double2 w[4][D];
+          hop_values<D, double, E1, false>(a, t, w);
+          store_spinor<D, double>(L.o, w, L.g, Vh + t);
+        }
+      }
+      if (!group_sync(cnt, due, nb, err, limit)) { status = YG_TIMEOUT; break; }
+      double acc = 0.0;
+      for (int k = 0; k < passes; k++) {
+        const int t = first + k * stride;
+        const bool live = t < Vh;
+        if (QUAD) {
+          double2 w[D];
+          long at;
+          hop_quad<D, double, E2, false>(e, live ? t : Vh - 1, live, w, at);
+          if (live) {
+#pragma unroll
+            for (int c = 0; c < D; c++) acc += finish(w[c], half, L.t, L.r, alpha, at + (long)c * Vh);
+          }
+        } else if (live) {
+          double2 w[4][D];
+          hop_values<D, double, E2, false>(e, t, w);
+#pragma unroll
+          for (int sp = 0; sp < 4; sp++)
+#pragma unroll
+            for (int c = 0; c < D; c++) acc += finish(w[sp][c], half, L.t, L.r, alpha, (long)(sp * D + c) * Vh + t);
+        }
+      }
+      double *part = half ? part_rr : part_pq;
+      acc = block_sum(acc);
+      if (threadIdx.x == 0) part[blockIdx.x] = acc;
+      if (!group_sync(cnt, due, nb, err, limit)) { status = YG_TIMEOUT; break; }
+      const double total = group_total(part, L.b0, nb);
+      if (!isfinite(total)) { status = YG_NONFINITE; break; }
+      if (half == 0) {
+        alpha = rr / total;
+      } else {
+        const double beta = total / rr;
+        rr = total;
+        for (int k = 0; k < passes; k++) {
+          const int t = first + k * stride;
+          if (t >= Vh) break;
+          const long at = (long)(QUAD ? (threadIdx.x & 3) * D : 0) * Vh + t;
+#pragma unroll
+          for (int c = 0; c < (QUAD ? D : 4 * D); c++) {
+            const long i = at + (long)c * Vh;
+            const double2 pv = L.p[i], rv = L.r[i];
+            double2 xv = L.x[i];
+            xv.x = fma(alpha, pv.x, xv.x);
+            xv.y = fma(alpha, pv.y, xv.y);
+            L.x[i] = xv;
+            L.p[i] = make_double2(fma(beta, pv.x, rv.x), fma(beta, pv.y, rv.y));
+          }
+        }
+      }
+    }
+    if (status != YG_OK || rr < L.target) break;
+    if (!group_sync(cnt, due, nb, err, limit)) status = YG_TIMEOUT;
+  }
+  if (lb == 0 && threadIdx.x == 0) {
+    out->iters = it;
+    out->status = status;
+    out->rr = rr;
+  }
 }
 
 // CLOV = 1: A_oo^-1 from the packed inverse blocks and A_ee from the clover term (d <= 6);
-// CLOV = 0: no clover term, A_oo = 1 and the (4+m)^2 diagonal.  Registers are capped for 3
-// resident CTAs per SM, so that a 16^4 lattice's group covers its 32768 even sites in one
-// pass of the grid (one site per thread).
+// CLOV = 0: no clover term, A_oo = 1 and the (4+m)^2 diagonal.
 template <int D, int CLOV>
-__global__ void __launch_bounds__(kThreads, 3) k_cg_batch(const BLat *lats, int n, double *part_pq, double *part_rr,
-                                                       unsigned *sync, int *err, BOut *out, long long limit) {
-  constexpr int E1 = CLOV ? EPI_CLOVPK : EPI_PLAIN, E2 = CLOV ? EPI_CLOVADD : EPI_AXPY;
+__global__ void __launch_bounds__(kThreads, 3) k_cg_batch(const __grid_constant__ BArgs args, double *part_pq,
+                                                       double *part_rr, unsigned *sync, int *err, BOut *out,
+                                                       long long limit) {
   int li = 0;
-  while (li + 1 < n && (int)blockIdx.x >= lats[li + 1].b0) li++;
-  const BLat &L = lats[li];
-  const int lb = blockIdx.x - L.b0;
-  const int first = lb * kThreads + threadIdx.x, stride = L.nb * kThreads;
-  const int Vh = L.s2a.g.Vh;
-  constexpr int NC = 4 * D;                          // complex words per site
-  unsigned *cnt = sync + 2 * li, *gen = cnt + 1;
-  double rr = L.rr0;
-  int it = 0, status = YG_OK;
-  // cg.cpp:151-153: a system solved by its initial guess returns 0 iterations
-  while (L.it0 == 0) {
-    ++it;
-    if (L.maxiter > 0 && it > L.maxiter) { it--; status = YG_MAXITER; break; }
-    for (int t = first; t < Vh; t += stride) step<D, E1>(L.s1a, t);
-    if (!group_sync(cnt, gen, L.nb, err, limit)) { status = YG_TIMEOUT; break; }
-    for (int t = first; t < Vh; t += stride) step<D, E2>(L.s2a, t);
-    if (!group_sync(cnt, gen, L.nb, err, limit)) { status = YG_TIMEOUT; break; }
-    for (int t = first; t < Vh; t += stride) step<D, E1>(L.s1b, t);
-    if (!group_sync(cnt, gen, L.nb, err, limit)) { status = YG_TIMEOUT; break; }
-    double acc = 0.0;
-    for (int t = first; t < Vh; t += stride) {
-      step<D, E2>(L.s2b, t);
-      double s = 0.0;                                // Re <p, q> of the site just written
-#pragma unroll 4
-      for (int k = 0; k < NC; k++) {
-        const long i = (long)k * Vh + t;
-        const double2 pv = L.p[i], qv = L.q[i];
-        s = fma(pv.x, qv.x, fma(pv.y, qv.y, s));
-      }
-      acc += s;
+  while (li + 1 < args.n && (int)blockIdx.x >= args.l[li + 1].b0) li++;
+  const BLat &L = args.l[li];
+  unsigned *cnt = sync + kSyncStride * li;
+  if constexpr (D <= kSiteMaxD) {
+    if (!L.quad) {
+      group_cg<D, CLOV, false>(L, part_pq, part_rr, cnt, err, out + li, limit);
+      return;
     }
-    acc = block_sum(acc);
-    if (threadIdx.x == 0) part_pq[blockIdx.x] = acc;
-    if (!group_sync(cnt, gen, L.nb, err, limit)) { status = YG_TIMEOUT; break; }
-    const double pq = group_total(part_pq, L.b0, L.nb);
-    if (!isfinite(pq)) { status = YG_NONFINITE; break; }
-    const double alpha = rr / pq;
-    acc = 0.0;
-    for (int t = first; t < Vh; t += stride) {
-      double s = 0.0;
-#pragma unroll 4
-      for (int k = 0; k < NC; k++) {
-        const long i = (long)k * Vh + t;
-        const double2 pv = L.p[i], qv = L.q[i];
-        double2 xv = L.x[i], rv = L.r[i];
-        xv.x = fma(alpha, pv.x, xv.x);
-        xv.y = fma(alpha, pv.y, xv.y);
-        rv.x = fma(-alpha, qv.x, rv.x);
-        rv.y = fma(-alpha, qv.y, rv.y);
-        L.x[i] = xv;
-        L.r[i] = rv;
-        s = fma(rv.x, rv.x, fma(rv.y, rv.y, s));
-      }
-      acc += s;
-    }
-    acc = block_sum(acc);
-    if (threadIdx.x == 0) part_rr[blockIdx.x] = acc;
-    if (!group_sync(cnt, gen, L.nb, err, limit)) { status = YG_TIMEOUT; break; }
-    const double rrn = group_total(part_rr, L.b0, L.nb);
-    if (!isfinite(rrn)) { status = YG_NONFINITE; break; }
-    const double beta = rrn / rr;
-    rr = rrn;
-    if (rr < L.target) break;
-    for (int t = first; t < Vh; t += stride) {
-#pragma unroll 4
-      for (int k = 0; k < NC; k++) {
-        const long i = (long)k * Vh + t;
-        const double2 pv = L.p[i], rv = L.r[i];
-        L.p[i] = make_double2(fma(beta, pv.x, rv.x), fma(beta, pv.y, rv.y));
-      }
-    }
-    if (!group_sync(cnt, gen, L.nb, err, limit)) { status = YG_TIMEOUT; break; }
   }
-  if (lb == 0 && threadIdx.x == 0) {
-    out[li].iters = it;
-    out[li].status = status;
-    out[li].rr = rr;
-  }
+  group_cg<D, CLOV, true>(L, part_pq, part_rr, cnt, err, out + li, limit);
 }
 
 template <int D, int CLOV>
-void launch_batch(int grid, cudaStream_t s, const BLat *lats, int n, double *part_pq, double *part_rr,
-                  unsigned *sync, int *err, BOut *out, long long limit) {
-  void *args[] = {(void *)&lats, (void *)&n, (void *)&part_pq, (void *)&part_rr, (void *)&sync, (void *)&err,
-                  (void *)&out, (void *)&limit};
+void launch_batch(int grid, cudaStream_t s, const BArgs &a, double *part_pq, double *part_rr, unsigned *sync, int *err,
+                  BOut *out, long long limit) {
+  void *args[] = {(void *)&a, (void *)&part_pq, (void *)&part_rr, (void *)&sync, (void *)&err, (void *)&out,
+                  (void *)&limit};
   YG_CUDA(cudaLaunchCooperativeKernel((const void *)k_cg_batch<D, CLOV>, dim3(grid), dim3(kThreads), args, 0, s));
   YG_LAUNCHED();
 }
@@ -235,31 +289,6 @@ int resident_blocks() {
     }                                                                                                             \
   } while (0)
 
-HopArgs<double> step_args(Lattice &L, bool first_step, double mass, const double *src, double *dst,
-                          const double *src2) {
-  HopArgs<double> a{};
-  a.g = L.g;
-  a.cfm1 = L.p.cf - 1.0;
-  a.U = L.links.as<double2>();
-  a.src = (const double2 *)src;
-  a.dst = (double2 *)dst;
-  a.n = (int)L.Vh;
-  if (first_step) {                          // schur_step1: odd output, A_oo^-1 (1/2 H src)
-    a.lo = (int)L.Vh;
-    a.coeff = 0.5;
-    if (L.p.clover) a.cpk = L.cpk64.as<double2>();
-  } else {                                   // schur_step2: even output, g5 (A_ee src2 - 1/2 H src)
-    a.lo = 0;
-    a.src2 = (const double2 *)src2;
-    a.coeff = -0.5;
-    a.g5 = 1;
-    a.zero_add_at_boundary = 1;
-    if (L.p.clover) { a.cl = L.clover.as<double2>(); a.diag = 4.0 + mass; }
-    else a.diag = (4.0 + mass) * (4.0 + mass);
-  }
-  return a;
-}
-
 }  // namespace
 
 bool batch_eligible(int n, Lattice *const *L, const yg_inv_par *par) {
@@ -277,13 +306,15 @@ bool batch_eligible(int n, Lattice *const *L, const yg_inv_par *par) {
 // with the engine's ordinary launches, then one persistent launch for all iterations.
 int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, double *const *xs, double *const *bs,
                            int *iters, long long wait_cycles) {
-  if (n < 1 || n > 64) throw Error(YG_ERR_ARG, "1..64 lattices");
+  if (n < 1 || n > kMaxLattices) throw Error(YG_ERR_ARG, "1..64 lattices");
   if (!batch_eligible(n, L, par))
     throw Error(YG_ERR_ARG, "the persistent batch solves Hphi_sq on even-odd lattices of one d (2, 3, 4 or 6), "
                             "all with or all without a clover term, without open/SF boundaries");
   const int d = L[0]->d;
   const bool clov = L[0]->p.clover;
-  std::vector<BLat> h(n);
+  BArgs args{};
+  args.n = n;
+  BLat *h = args.l;
   long vol = 0;
   for (int i = 0; i < n; i++) vol += L[i]->Vh;
   int grid_max = 0;
@@ -305,45 +336,48 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
     const double norm = blas_sqnorm(l, bs[i], lo, cnt);
     const double rr = blas_sqnorm(l, r, lo, cnt);
     BLat &b = h[i];
-    b.s1a = step_args(l, true, mass, p, o, nullptr);
-    b.s2a = step_args(l, false, mass, o, t, p);
-    b.s1b = step_args(l, true, mass, t, o, nullptr);
-    b.s2b = step_args(l, false, mass, o, q, t);
+    b.g = l.g;
+    b.U = l.links.as<double2>();
+    b.cl = l.clover.as<double2>();
+    b.cpk = l.cpk64.as<double2>();
+    b.diag = clov ? 4.0 + mass : (4.0 + mass) * (4.0 + mass);
+    b.t = (double2 *)t;
+    b.o = (double2 *)o;
     b.x = (double2 *)xs[i];
     b.r = (double2 *)r;
     b.p = (double2 *)p;
-    b.q = (double2 *)q;
     b.maxiter = par[i].maxiter;
     b.target = norm * par[i].prec;
     b.rr0 = rr;
     b.it0 = rr < b.target ? -1 : 0;
-    // blocks in proportion to the even volume, at least one, at most one per 128 sites
-    const long share = (long)((double)grid_max * (double)l.Vh / (double)vol);
-    b.nb = (int)std::max<long>(1, std::min<long>(share, nblk(l.Vh, kThreads)));
+    // blocks in proportion to the even volume, at least one, and no more than the passes over the
+    // sites need (fewer blocks make a cheaper barrier)
+    const long share = std::max(1L, (long)((double)grid_max * (double)l.Vh / (double)vol));
+    b.quad = d > kSiteMaxD || l.Vh <= kQuadSites;
+    const long tiles = nblk(l.Vh, b.quad ? kThreads / 4 : kThreads), passes = (tiles + share - 1) / share;
+    b.nb = (int)((tiles + passes - 1) / passes);
     b.b0 = b0;
     b0 += b.nb;
     YG_CUDA(cudaStreamSynchronize(l.stream));
   }
   const int grid = b0;
   if (grid > grid_max) throw Error(YG_ERR_ARG, "block groups exceed the resident grid");
-  // one device allocation: lattice records, partials, barrier words, error flag, results
-  const size_t off_part = ((sizeof(BLat) * n + 255) / 256) * 256;
-  const size_t off_sync = off_part + 2 * sizeof(double) * grid;
-  const size_t off_err = off_sync + ((sizeof(unsigned) * 2 * n + 15) / 16) * 16;
+  // one device buffer: partials, barrier counters, error flag, results
+  const size_t off_sync = (2 * sizeof(double) * grid + 127) / 128 * 128;
+  const size_t off_err = off_sync + sizeof(unsigned) * kSyncStride * n;
   const size_t off_out = off_err + 16;
   const size_t bytes = off_out + sizeof(BOut) * n;
-  DevBuf buf;
-  buf.alloc(bytes);
-  char *base = buf.as<char>();
+  L[0]->cg_work.alloc(bytes);            // kept: an allocation would synchronise the device on every solve
+  char *base = L[0]->cg_work.as<char>();
   cudaStream_t s = L[0]->stream;
   int err = 0;
   std::vector<BOut> res(n);
+  std::lock_guard<std::mutex> one(g_persistent);
   try {
     YG_CUDA(cudaMemsetAsync(base, 0, bytes, s));
-    YG_CUDA(cudaMemcpyAsync(base, h.data(), sizeof(BLat) * n, cudaMemcpyHostToDevice, s));
     const long long limit = wait_cycles > 0 ? wait_cycles : kDefaultWait;
-    double *part = reinterpret_cast<double *>(base + off_part);
-    YG_BATCH_D(d, clov, launch_batch<BD, BC>(grid, s, reinterpret_cast<const BLat *>(base), n, part, part + grid,
+    double *part = reinterpret_cast<double *>(base);
+    YG_BATCH_D(d, clov, launch_batch<BD, BC>(grid, s, args, part, part + grid,
                                              reinterpret_cast<unsigned *>(base + off_sync),
                                              reinterpret_cast<int *>(base + off_err),
                                              reinterpret_cast<BOut *>(base + off_out), limit));
@@ -352,10 +386,8 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
     YG_CUDA(cudaStreamSynchronize(s));
   } catch (...) {
     cudaStreamSynchronize(s);
-    buf.release();
     throw;
   }
-  buf.release();
   int worst = YG_OK;
   for (int i = 0; i < n; i++) {
     iters[i] = res[i].iters;

@@ -71,6 +71,8 @@ struct Lattice {
   DevBuf tables;    // basis / generators
   ReprTables rt{};
 
+  DevBuf cg_work;   // records, partials and barrier words of the persistent CG (yg_batch.cu)
+
   // reduction scratch: per-block partial sums + result
   DevBuf red_partial;
   DevBuf red_result;

@@ -55,8 +55,9 @@ void check_finite(double v, const char *what) {
 
 }  // namespace
 
-// cg_inverter, cg.cpp:132-202
-int cg(Lattice &L, const yg_inv_par &par, double *x, double *b, int *iters) {
+// cg_inverter, cg.cpp:132-202, one launch per operator step and vector pass, with two host round
+// trips an iteration: any operator, representation and boundary condition
+static int cg_launches(Lattice &L, const yg_inv_par &par, double *x, double *b, int *iters) {
   Ctx c(L);
   double *r = L.scratch_field(3), *p = L.scratch_field(4), *q = L.scratch_field(5);
   c.copy(p, x);
@@ -83,6 +84,22 @@ int cg(Lattice &L, const yg_inv_par &par, double *x, double *b, int *iters) {
   log_line(par, "cg", it, rr / norm);
   *iters = it;
   return status;
+}
+
+// cg_inverter.  The systems the persistent kernel covers (Hphi_sq with even-odd preconditioning, no
+// open or SF slices, d = 2, 3, 4, 6) iterate wholly on the device while the launches and host round
+// trips of an iteration weigh more than its data; us an iteration, launches / persistent:
+//   d = 3: 4^4 86 / 28, 8^4 85 / 29, 12^4 91 / 61, 16^4 130 / 107, 32 x 16^3 234 / 250, 32^4 1146 / 1300;
+//   d = 2: 16^4 93 / 45;  d = 6: 8^4 139 / 61, 16^4 309 / 442
+constexpr long kPersistentColours = 100000;     // even sites times d
+
+int cg(Lattice &L, const yg_inv_par &par, double *x, double *b, int *iters) {
+  Lattice *l = &L;
+  if (L.Vh * L.d > kPersistentColours || !batch_eligible(1, &l, &par)) return cg_launches(L, par, x, b, iters);
+  const int st = cg_lattices_persistent(1, &l, &par, &x, &b, iters, 0);
+  if (st == YG_NONFINITE) throw Error(YG_NONFINITE, "non-finite value in cg");
+  if (st == YG_TIMEOUT) throw Error(YG_TIMEOUT, "a barrier wait of the persistent CG ran out");
+  return st;
 }
 
 // No reference counterpart: independent cg_inverter solves on lattices of any sizes at once.
