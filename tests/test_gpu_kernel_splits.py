@@ -83,3 +83,30 @@ def test_persistent_cg(name, dims):
     assert lat.cg_inverter("Hphi_sq", 0.2, 1e-20, x, b) == 0
     lat.spinor_zero(x)
     assert lat.cg_inverter("Hphi_sq", 0.2, 1e-22, x, b, maxiter=3) == 3 and lat.last_status == 4
+
+
+@pytest.mark.parametrize("channels", [(1, 8, 8, 1), (1, 16, 16, 1)])
+def test_network_on_ragged_tiles(channels):
+    """432 even sites: 6.75 tiles of 64, so one tile straddles the parities and takes all nine paths,
+    the others leave out the paths that carry nothing.  BF16 operands: 2e-2 as in the layer tests."""
+    from oracle import ptc_oracle as po
+    from yahmc_b200 import Ptc
+    lat, O, rng = make_pair("su3_fund_ap", (4, 6, 6, 6), seed=24)
+    net = Ptc(lat, channels)
+    Ws = [(rng.standard_normal(s) + 1j * rng.standard_normal(s)) / np.sqrt(2 * 9 * 4 * s[2]) for s in net.shapes()]
+    net.set_weights(Ws)
+    pairs = []
+    for _ in range(2):
+        r, e = source(O, rng), source(O, rng)
+        r[O.Vh:] = 0
+        e[O.Vh:] = 0
+        pairs.append((r, e))
+    onet = po.Net(Ws)
+    d, s = lat.field(), lat.field(pairs[0][0])
+    net.apply(d, s)
+    assert rel(lat.download(d)[:O.Vh], po.apply_even(O, onet, pairs[0][0][:O.Vh])) < 2e-2
+    loss, grads = net.gradient([(lat.field(r), lat.field(e)) for r, e in pairs])
+    lo, go = po.loss_and_grads(O, onet, [(r[:O.Vh], e[:O.Vh]) for r, e in pairs])
+    assert abs(loss - lo) < 2e-2 * lo
+    for g, h in zip(grads, go):
+        assert rel(g, h) < 2e-2

@@ -100,6 +100,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase) {
   return false;
 }
 
+// bulk copy of `bytes` (a multiple of 16) into shared memory, completing on the barrier
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t mbar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(mbar)
+               : "memory");
+}
+
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -138,13 +146,13 @@ struct PtcArgs {
   float *part;              // wgrad: per-CTA partial weight gradients
   int *err;                 // bounded-wait failures
   int V;
+  int nout;                 // sites of the output that are wanted: [0, nout), V or the even half
+  int in_even;              // the input vanishes on odd sites: a site's own path or its eight hops carry nothing
 };
 
-// site id and its neighbour along path p (p = 0 itself), and the link that transports from it
-__device__ __forceinline__ int path_site(const Geom &g, int id, int p) {
+// the neighbour of site id (coordinates c) along path p (p = 0 itself)
+__device__ __forceinline__ int path_site(const Geom &g, int id, const int c[4], int p) {
   if (p == 0) return id;
-  int c[4];
-  coords_of(g, id, c);
   return p <= 4 ? neighbour(g, c, p - 1, +1) : neighbour(g, c, p - 5, -1);
 }
 
@@ -219,57 +227,75 @@ __device__ __forceinline__ void transport_block(float2 (&y)[4][3], const Block &
 // ---------------------------------------------------------------- forward layer
 // grid: one CTA per tile of 64 sites.  CI input channels (1 or a multiple of 2), CO output
 // channels (2 * CO * 4 <= 128 rows).  KP = columns of one path's chunk (2 CI 4, padded to 16).
+//
+// Bound by the latency of the gathers (two CTAs an SM, by tensor memory), so the paths are pipelined:
+// while the tensor core multiplies one path's operands the threads gather the next path into the other
+// buffer, and the packed weights arrive by bulk copy.  With C = 16 two buffers would leave one CTA an
+// SM, so there the gather waits for the product.  A path that carries nothing on the whole tile
+// (in_even, tiles of one parity) is left out.
+template <int CI> struct LayerBufs { static constexpr int value = CI <= 8 ? 2 : 1; };
+
 template <int CI, int CO>
 __global__ void __launch_bounds__(kThreads, 1) k_ptc_layer(PtcArgs a) {
   constexpr int KP = ((2 * CI * 4 + 15) / 16) * 16;
   constexpr int PAIRS = CI * 4;                          // (channel, spin) pairs per site
+  constexpr int NBUF = LayerBufs<CI>::value;
+  constexpr uint32_t ABYTES = kM * KP * 2, BBYTES = kN * KP * 2;
+  constexpr uint32_t AUSED = CO * KP * 16;               // rows 0 .. 8 CO - 1 of a chunk, the others are zero
   extern __shared__ __align__(1024) unsigned char sm[];
-  unsigned char *sA = sm;                                // kM x KP
-  unsigned char *sB = sm + kM * KP * 2;                  // kN x KP
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(sB + kN * KP * 2);
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + 1);
-  __shared__ int s_site[kTileSites], s_nbr[kTileSites];
+  unsigned char *sA = sm;                                // NBUF x kM x KP
+  unsigned char *sB = sm + NBUF * ABYTES;                // NBUF x kN x KP
+  uint64_t *mbar = reinterpret_cast<uint64_t *>(sB + NBUF * BBYTES);    // [0, NBUF) products, then weights
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + 2 * NBUF);
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int t0 = blockIdx.x * kTileSites;
   if (warp == 0) tmem_alloc(smem_u32(tslot), kTmemCols);
-  if (tid == 0) mbar_init(smem_u32(mbar));
+  if (tid == 0)
+    for (int i = 0; i < 2 * NBUF; i++) mbar_init(smem_u32(mbar + i));
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  // zero once: the rows of A beyond the outputs, the padding columns of B (CI = 1: columns 8..15)
+  for (int buf = 0; buf < NBUF; buf++)
+    for (int e = AUSED / 16 + tid; e < (int)(ABYTES / 16); e += kThreads)
+      reinterpret_cast<uint4 *>(sA + buf * ABYTES)[e] = make_uint4(0, 0, 0, 0);
+  if constexpr (KP > 2 * PAIRS) {
+    for (int e = tid; e < NBUF * kN * (KP - 2 * PAIRS); e += kThreads) {
+      const int r = (e / (KP - 2 * PAIRS)) % kN, k = 2 * PAIRS + e % (KP - 2 * PAIRS), buf = e / (kN * (KP - 2 * PAIRS));
+      put_bf16(sB + buf * BBYTES, kmajor_off(r, k, KP), 0.f);
+    }
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tslot;
-  bool ok = true;
+  bool ok = true, good = true;      // the block's, and this thread's waits
 
-  // zero the padding columns of B once (CI = 1: columns 8..15 stay zero)
-  if constexpr (KP > 2 * PAIRS) {
-    for (int e = tid; e < kN * (KP - 2 * PAIRS); e += kThreads) {
-      const int r = e / (KP - 2 * PAIRS), k = 2 * PAIRS + e % (KP - 2 * PAIRS);
-      put_bf16(sB, kmajor_off(r, k, KP), 0.f);
-    }
+  constexpr int NPART = kThreads / kTileSites;
+  const int j = tid % kTileSites, part = tid / kTileSites;
+  const int id = t0 + j;
+  const bool live = id < a.nout;
+  int c[4];
+  coords_of(a.g, live ? id : 0, c);
+  int p0 = 0, np = kPaths;                               // paths p0 .. p0 + np - 1
+  if (a.in_even) {
+    if (t0 + kTileSites <= a.g.Vh) np = 1;
+    else if (t0 >= a.g.Vh) { p0 = 1; np = kPaths - 1; }
   }
 
-  for (int p = 0; p < kPaths && ok; p++) {
-    // A chunk of path p: a straight copy of the packed operand
-    {
-      const uint4 *src = reinterpret_cast<const uint4 *>(a.A + (long)p * kM * KP);
-      uint4 *dst = reinterpret_cast<uint4 *>(sA);
-      for (int e = tid; e < kM * KP * 2 / 16; e += kThreads) dst[e] = __ldg(src + e);
-    }
+#pragma unroll 1
+  for (int i = 0; i < np && ok; i++) {
+    const int p = p0 + i, buf = i % NBUF;
+    const uint32_t mma_bar = smem_u32(mbar + buf), w_bar = smem_u32(mbar + NBUF + buf);
+    unsigned char *B = sB + buf * BBYTES;
+    // the buffers' last product is done; a wait that runs out ends the loop for all at the next barrier
+    if (i >= NBUF) good = mbar_wait(mma_bar, (uint32_t)((i / NBUF - 1) & 1)) && good;
+    if (tid == 0 && good) bulk_load(smem_u32(sA + buf * ABYTES), a.A + (long)p * kM * KP, AUSED, w_bar);
     // B chunk: the transported inputs of the tile's sites.  Thread (site j, part) takes the
-    // channels part, part + NPART, ...; a one-channel input is split by spin pairs instead.
-    if (tid < kTileSites) {
-      const int id = t0 + tid;
-      s_site[tid] = id < a.V ? id : -1;
-      s_nbr[tid] = id < a.V ? path_site(a.g, id, p) : -1;
-    }
-    __syncthreads();
-    {
-      constexpr int NPART = kThreads / kTileSites;
-      const int j = tid % kTileSites, part = tid / kTileSites;
-      const int id = s_site[j], nid = s_nbr[j];
+    // channels part, part + NPART, ...; a one-channel input is gathered by part 0.
+    if (CI >= NPART || part == 0) {
+      const int nid = live ? path_site(a.g, id, c, p) : 0;
       float2 u[9];
-      if (id >= 0 && p > 0) path_link(a, id, nid, p, u);
+      if (live && p > 0) path_link(a, id, nid, p, u);
       constexpr int NCH = CI >= NPART ? CI / NPART : 1;     // channels per thread
       constexpr int CB = NCH < 4 ? NCH : 4;                  // gathered together
 #pragma unroll 1
@@ -278,10 +304,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_ptc_layer(PtcArgs a) {
 #pragma unroll
         for (int q = 0; q < CB; q++) {
           const int ch = CI >= NPART ? part + NPART * (c0 + q) : 0;
-          if (id >= 0) load_block(f[q], a.in, (long)ch * a.V + nid);
+          if (live) load_block(f[q], a.in, (long)ch * a.V + nid);
           else
 #pragma unroll
-            for (int i = 0; i < 6; i++) f[q].w[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int k = 0; k < 6; k++) f[q].w[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int q = 0; q < CB; q++) {
@@ -289,42 +315,36 @@ __global__ void __launch_bounds__(kThreads, 1) k_ptc_layer(PtcArgs a) {
           float2 y[4][3];
           if (p == 0) transport_block<true>(y, f[q], u);
           else transport_block<false>(y, f[q], u);
-          if (CI >= NPART) {
 #pragma unroll
-            for (int c = 0; c < 3; c++) {
-              const int r = c * kTileSites + j;
-              put_bf16x4(sB, kmajor_off(r, ch * 4, KP), y[0][c].x, y[1][c].x, y[2][c].x, y[3][c].x);
-              put_bf16x4(sB, kmajor_off(r, PAIRS + ch * 4, KP), y[0][c].y, y[1][c].y, y[2][c].y, y[3][c].y);
-            }
-          } else if (part == 0) {
-            // one input channel: columns 0..3 real, 4..7 imaginary, written by part 0
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-              const int r = c * kTileSites + j;
-              put_bf16x4(sB, kmajor_off(r, 0, KP), y[0][c].x, y[1][c].x, y[2][c].x, y[3][c].x);
-              put_bf16x4(sB, kmajor_off(r, 4, KP), y[0][c].y, y[1][c].y, y[2][c].y, y[3][c].y);
-            }
+          for (int cl = 0; cl < 3; cl++) {
+            const int r = cl * kTileSites + j;
+            put_bf16x4(B, kmajor_off(r, ch * 4, KP), y[0][cl].x, y[1][cl].x, y[2][cl].x, y[3][cl].x);
+            put_bf16x4(B, kmajor_off(r, PAIRS + ch * 4, KP), y[0][cl].y, y[1][cl].y, y[2][cl].y, y[3][cl].y);
           }
         }
       }
     }
     fence_async_smem();
     tc_fence_before();
-    __syncthreads();
-    if (tid == 0) {
+    ok = __syncthreads_and(good);
+    if (tid == 0 && ok) {
+      good = mbar_wait(w_bar, (uint32_t)((i / NBUF) & 1));
       tc_fence_after();
-      const uint32_t aa = smem_u32(sA), bb = smem_u32(sB);
+      if (good) {
+        const uint32_t aa = smem_u32(sA + buf * ABYTES), bb = smem_u32(B);
 #pragma unroll
-      for (int kk = 0; kk < KP / 16; kk++)
-        mma_bf16(tmem, smem_desc(aa + kk * 256, KP), smem_desc(bb + kk * 256, KP), idesc_bf16(kM, kN),
-                 (p > 0 || kk > 0) ? 1u : 0u);
-      mma_commit(smem_u32(mbar));
+        for (int kk = 0; kk < KP / 16; kk++)
+          mma_bf16(tmem, smem_desc(aa + kk * 256, KP), smem_desc(bb + kk * 256, KP), idesc_bf16(kM, kN),
+                   (i > 0 || kk > 0) ? 1u : 0u);
+        mma_commit(mma_bar);
+      }
     }
-    ok = mbar_wait(smem_u32(mbar), (uint32_t)(p & 1));
-    if (!ok && tid == 0) atomicExch(a.err, 1);
-    tc_fence_after();
-    ok = __syncthreads_and(ok);
   }
+  // the last product of each buffer: products complete in order, so the last one implies the others
+  if (ok && good) good = mbar_wait(smem_u32(mbar + (np - 1) % NBUF), (uint32_t)(((np - 1) / NBUF) & 1));
+  if (!good) atomicExch(a.err, 1);
+  tc_fence_after();
+  ok = __syncthreads_and(ok && good);
 
   if (ok) {
     // epilogue: accumulator row m = (o, s) real part (m < 4 CO) or imaginary part
@@ -344,7 +364,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_ptc_layer(PtcArgs a) {
     __syncthreads();
     for (int e = tid; e < kTileSites * CO; e += kThreads) {
       const int j = e % kTileSites, o = e / kTileSites;
-      if (t0 + j >= a.V) continue;
+      if (t0 + j >= a.nout) continue;
       float4 w[6];
       float *wf = reinterpret_cast<float *>(w);
 #pragma unroll
@@ -367,31 +387,41 @@ __global__ void __launch_bounds__(kThreads, 1) k_ptc_layer(PtcArgs a) {
 // ---------------------------------------------------------------- weight gradient
 // dW_p^T[(i, s'), (o, s)] = sum_n X_p[(i, s'), n] conj(G[(o, s), n]) as a real product
 //   [C_re | C_im] = [X_re | X_im] [[G_re^T, -G_im^T]; [G_im^T, G_re^T]]
-// A (rows (i, s'), padded to 128; columns (n re | n im), 2 kN) and B (rows the 2 CO 4 columns
-// of [C_re | C_im], padded to NB; same K) in shared memory; the CTA accumulates its tiles for
-// a group of paths in tensor memory (NB columns per path) and writes one partial per path.
-template <int CI, int CO, int PG>
-__global__ void __launch_bounds__(kThreads, 1) k_ptc_wgrad(PtcArgs a, int ntiles) {
+// A (rows (path, i, s'), padded to 128; columns (n re | n im), 2 kN) and B (rows the 2 CO 4 columns
+// of [C_re | C_im], padded to NB; same K) in shared memory: PG paths share the 128 rows of one product
+// (9, 3 or 2 paths for 1, 8 or 16 input channels), each gathered by its own threads, where one path at
+// a time left 3/4 of the rows empty and 128 threads a SM.  The CTA accumulates its tiles in tensor
+// memory and writes one partial per path.
+template <int CI> struct WgradCfg {
+  static constexpr int PG = CI == 1 ? 9 : CI == 8 ? 3 : 2;      // paths per product
+  static constexpr int parts = CI == 1 ? 1 : 2;                 // threads per path and site
+  static constexpr int threads = PG * parts * kTileSites;
+  static constexpr int groups = (kPaths + PG - 1) / PG;
+};
+
+template <int CI, int CO>
+__global__ void __launch_bounds__(WgradCfg<CI>::threads, 1) k_ptc_wgrad(PtcArgs a, int ntiles) {
+  using Cfg = WgradCfg<CI>;
+  constexpr int PG = Cfg::PG, NT = Cfg::threads;
   constexpr int KW = 2 * kN;                              // reduction columns per tile
-  constexpr int NB = ((2 * CO * 4 + 15) / 16) * 16;       // GEMM columns per path
+  constexpr int NB = ((2 * CO * 4 + 15) / 16) * 16;       // GEMM columns
   constexpr int PAIRS = CI * 4, OPAIRS = CO * 4;
   extern __shared__ __align__(1024) unsigned char sm[];
   unsigned char *sA = sm;                                 // kM x KW (transported inputs)
   unsigned char *sB = sm + kM * KW * 2;                   // NB x KW (output gradients)
   uint64_t *mbar = reinterpret_cast<uint64_t *>(sB + NB * KW * 2);
   uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + 1);
-  __shared__ int s_site[kTileSites], s_nbr[kTileSites];
-  constexpr int cols = NB * PG <= 32 ? 32 : NB * PG <= 64 ? 64 : NB * PG <= 128 ? 128 : NB * PG <= 256 ? 256 : 512;
-  static_assert(NB * PG <= 512, "tensor memory columns");
+  constexpr int cols = NB <= 32 ? 32 : NB <= 64 ? 64 : 128;
+  static_assert(PG * PAIRS <= kM && NB <= 128, "one product per tile");
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int p0 = blockIdx.y * PG;
   if (warp == 0) tmem_alloc(smem_u32(tslot), cols);
   if (tid == 0) mbar_init(smem_u32(mbar));
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  // rows of A beyond the input pairs stay zero
-  for (int e = tid; e < (kM - PAIRS) * KW; e += kThreads) put_bf16(sA, kmajor_off(PAIRS + e / KW, e % KW, KW), 0.f);
-  for (int e = tid; e < (NB - 2 * OPAIRS) * KW; e += kThreads)
+  // rows of A beyond the paths' input pairs stay zero (the last group of two paths has one)
+  for (int e = tid; e < kM * KW * 2 / 16; e += NT) reinterpret_cast<uint4 *>(sA)[e] = make_uint4(0, 0, 0, 0);
+  for (int e = tid; e < (NB - 2 * OPAIRS) * KW; e += NT)
     put_bf16(sB, kmajor_off(2 * OPAIRS + e / KW, e % KW, KW), 0.f);
   tc_fence_before();
   __syncthreads();
@@ -399,15 +429,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_ptc_wgrad(PtcArgs a, int ntiles
   const uint32_t tmem = *tslot;
   bool ok = true;
   uint32_t phase = 0;
-  bool first = true;
+  const int j = tid % kTileSites, part = (tid / kTileSites) % Cfg::parts, pp = tid / (kTileSites * Cfg::parts);
+  const int p = p0 + pp;
 
   for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
     const int t0 = tile * kTileSites;
     // B: the output gradients of the tile (the same for every path), site blocks of gin
-    for (int e = tid; e < kTileSites * CO; e += kThreads) {
-      const int j = e % kTileSites, o = e / kTileSites, id = t0 + j;
+    for (int e = tid; e < kTileSites * CO; e += NT) {
+      const int jj = e % kTileSites, o = e / kTileSites, id = t0 + jj;
       Block gb;
-      if (id < a.V) load_block(gb, a.gin, (long)o * a.V + id);
+      if (id < a.nout) load_block(gb, a.gin, (long)o * a.V + id);
       else
 #pragma unroll
         for (int i = 0; i < 6; i++) gb.w[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -416,94 +447,82 @@ __global__ void __launch_bounds__(kThreads, 1) k_ptc_wgrad(PtcArgs a, int ntiles
 #pragma unroll
         for (int c = 0; c < 3; c++) {
           const float2 gv = blk_c(gb, sp, c);
-          const int os = o * 4 + sp, n = c * kTileSites + j;
+          const int os = o * 4 + sp, n = c * kTileSites + jj;
           put_bf16(sB, kmajor_off(os, n, KW), gv.x);
           put_bf16(sB, kmajor_off(os, kN + n, KW), gv.y);
           put_bf16(sB, kmajor_off(OPAIRS + os, n, KW), -gv.y);
           put_bf16(sB, kmajor_off(OPAIRS + os, kN + n, KW), gv.x);
         }
     }
-    for (int pp = 0; pp < PG && ok; pp++) {
-      const int p = p0 + pp;
-      if (tid < kTileSites) {
-        const int id = t0 + tid;
-        s_site[tid] = id < a.V ? id : -1;
-        s_nbr[tid] = id < a.V ? path_site(a.g, id, p) : -1;
-      }
-      __syncthreads();
-      {
-        constexpr int NPART = kThreads / kTileSites;
-        const int j = tid % kTileSites, part = tid / kTileSites;
-        const int id = s_site[j], nid = s_nbr[j];
-        float2 u[9];
-        if (id >= 0 && p > 0) path_link(a, id, nid, p, u);
-        constexpr int NCH = CI >= NPART ? CI / NPART : 1;
-        constexpr int CB = NCH < 4 ? NCH : 4;
+    if (p < kPaths) {
+      const int id = t0 + j;
+      int c[4];
+      coords_of(a.g, id < a.nout ? id : 0, c);
+      const bool live = id < a.nout && !(a.in_even && (p == 0) != (id < a.g.Vh));
+      const int nid = live ? path_site(a.g, id, c, p) : 0;
+      float2 u[9];
+      if (live && p > 0) path_link(a, id, nid, p, u);
+      constexpr int NCH = CI / Cfg::parts;
+      constexpr int CB = NCH < 4 ? NCH : 4;
 #pragma unroll 1
-        for (int c0 = 0; c0 < NCH; c0 += CB) {
-          Block f[CB];
+      for (int c0 = 0; c0 < NCH; c0 += CB) {
+        Block f[CB];
 #pragma unroll
-          for (int q = 0; q < CB; q++) {
-            const int ch = CI >= NPART ? part + NPART * (c0 + q) : 0;
-            if (id >= 0) load_block(f[q], a.in, (long)ch * a.V + nid);
-            else
+        for (int q = 0; q < CB; q++) {
+          const int ch = part + Cfg::parts * (c0 + q);
+          if (live) load_block(f[q], a.in, (long)ch * a.V + nid);
+          else
 #pragma unroll
-              for (int i = 0; i < 6; i++) f[q].w[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-          }
+            for (int i = 0; i < 6; i++) f[q].w[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
 #pragma unroll
-          for (int q = 0; q < CB; q++) {
-            const int ch = CI >= NPART ? part + NPART * (c0 + q) : 0;
-            if (CI < NPART && part != 0) continue;
-            float2 y[4][3];
-            if (p == 0) transport_block<true>(y, f[q], u);
-            else transport_block<false>(y, f[q], u);
+        for (int q = 0; q < CB; q++) {
+          const int ch = part + Cfg::parts * (c0 + q);
+          float2 y[4][3];
+          if (p == 0 || !live) transport_block<true>(y, f[q], u);
+          else transport_block<false>(y, f[q], u);
 #pragma unroll
-            for (int sp = 0; sp < 4; sp++)
+          for (int sp = 0; sp < 4; sp++)
 #pragma unroll
-              for (int c = 0; c < 3; c++) {
-                const int n = c * kTileSites + j, row = ch * 4 + sp;
-                put_bf16(sA, kmajor_off(row, n, KW), y[sp][c].x);
-                put_bf16(sA, kmajor_off(row, kN + n, KW), y[sp][c].y);
-              }
-          }
+            for (int cl = 0; cl < 3; cl++) {
+              const int n = cl * kTileSites + j, row = pp * PAIRS + ch * 4 + sp;
+              put_bf16(sA, kmajor_off(row, n, KW), y[sp][cl].x);
+              put_bf16(sA, kmajor_off(row, kN + n, KW), y[sp][cl].y);
+            }
         }
       }
-      fence_async_smem();
-      tc_fence_before();
-      __syncthreads();
-      if (tid == 0) {
-        tc_fence_after();
-        const uint32_t aa = smem_u32(sA), bb = smem_u32(sB);
-#pragma unroll 4
-        for (int kk = 0; kk < KW / 16; kk++)
-          mma_bf16(tmem + pp * NB, smem_desc(aa + kk * 256, KW), smem_desc(bb + kk * 256, KW), idesc_bf16(kM, NB),
-                   (!first || kk > 0) ? 1u : 0u);
-        mma_commit(smem_u32(mbar));
-      }
-      ok = mbar_wait(smem_u32(mbar), phase);
-      phase ^= 1u;
-      if (!ok && tid == 0) atomicExch(a.err, 1);
-      tc_fence_after();
-      ok = __syncthreads_and(ok);
-      if (pp == PG - 1) first = false;
     }
-    // the first tile initialised each path's accumulator (first flips after the last path)
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      tc_fence_after();
+      const uint32_t aa = smem_u32(sA), bb = smem_u32(sB);
+#pragma unroll 4
+      for (int kk = 0; kk < KW / 16; kk++)
+        mma_bf16(tmem, smem_desc(aa + kk * 256, KW), smem_desc(bb + kk * 256, KW), idesc_bf16(kM, NB),
+                 (tile != (int)blockIdx.x || kk > 0) ? 1u : 0u);
+      mma_commit(smem_u32(mbar));
+    }
+    ok = mbar_wait(smem_u32(mbar), phase);
+    phase ^= 1u;
+    if (!ok && tid == 0) atomicExch(a.err, 1);
+    tc_fence_after();
+    ok = __syncthreads_and(ok);
   }
 
-  if (ok) {
-    // row m = (i, s') (m < PAIRS), column pp * NB + j: j < 4 CO the real part of dW^T[(i,s'), (o,s)],
-    // 4 CO <= j < 8 CO its imaginary part.  part[(blockIdx.x * 9 + p) * kM * NB + m * NB + j]
-    const int m = warp * 32 + (tid & 31);
-    for (int pp = 0; pp < PG; pp++) {
-      for (int cb = 0; cb < (NB + 31) / 32; cb++) {
-        float v[32];
-        tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + pp * NB + cb * 32, v);
-        if (m < PAIRS) {
-          float *dst = a.part + ((long)blockIdx.x * kPaths + p0 + pp) * kM * NB + (long)m * NB + cb * 32;
+  if (ok && warp < 4) {
+    // row r = (path, i, s'), column j: j < 4 CO the real part of dW^T[(i,s'), (o,s)], 4 CO <= j < 8 CO
+    // its imaginary part.  part[(blockIdx.x * 9 + p) * kM * NB + (i,s') * NB + j]
+    const int r = warp * 32 + (tid & 31), pr = p0 + r / PAIRS;
+    for (int cb = 0; cb < (NB + 31) / 32; cb++) {
+      float v[32];
+      tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + cb * 32, v);
+      if (r < PG * PAIRS && pr < kPaths) {
+        float *dst = a.part + ((long)blockIdx.x * kPaths + pr) * kM * NB + (long)(r % PAIRS) * NB + cb * 32;
 #pragma unroll
-          for (int i = 0; i < 32; i++)
-            if (cb * 32 + i < NB) dst[i] = v[i];
-        }
+        for (int i = 0; i < 32; i++)
+          if (cb * 32 + i < NB) dst[i] = v[i];
       }
     }
   }
@@ -641,7 +660,9 @@ std::vector<double> adjoint_weights(const std::vector<double> &w, int ci, int co
 // columns and no allocation has to wait
 constexpr size_t kMinSmem = 100 * 1024;
 template <int CI, int CO>
-size_t layer_smem() { return std::max(kMinSmem, (size_t)kM * kp_of(CI) * 2 + (size_t)kN * kp_of(CI) * 2 + 16); }
+size_t layer_smem() {
+  return std::max(kMinSmem, (size_t)LayerBufs<CI>::value * ((size_t)(kM + kN) * kp_of(CI) * 2 + 16) + 16);
+}
 template <int CI, int CO>
 size_t wgrad_smem() { return (size_t)kM * 2 * kN * 2 + (size_t)(((2 * CO * 4 + 15) / 16) * 16) * 2 * kN * 2 + 16; }
 
@@ -649,19 +670,17 @@ template <int CI, int CO>
 void run_layer(Lattice &L, const PtcArgs &a) {
   const size_t sm = layer_smem<CI, CO>();
   YG_CUDA(cudaFuncSetAttribute(k_ptc_layer<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  k_ptc_layer<CI, CO><<<nblk(L.V, kTileSites), kThreads, sm, L.stream>>>(a);
+  k_ptc_layer<CI, CO><<<nblk(a.nout, kTileSites), kThreads, sm, L.stream>>>(a);
   YG_LAUNCHED();
 }
-
-constexpr int kPathGroup = 3;   // paths per wgrad CTA (3 x 128 accumulator columns)
 
 template <int CI, int CO>
 int run_wgrad(Lattice &L, const PtcArgs &a, int sms) {
   const size_t sm = wgrad_smem<CI, CO>();
-  YG_CUDA(cudaFuncSetAttribute(k_ptc_wgrad<CI, CO, kPathGroup>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  const int ntiles = nblk(L.V, kTileSites);
-  const int gx = std::min(ntiles, sms);
-  k_ptc_wgrad<CI, CO, kPathGroup><<<dim3(gx, kPaths / kPathGroup), kThreads, sm, L.stream>>>(a, ntiles);
+  YG_CUDA(cudaFuncSetAttribute(k_ptc_wgrad<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  const int ntiles = nblk(a.nout, kTileSites);
+  const int gx = std::min(ntiles, std::max(1, sms / WgradCfg<CI>::groups));     // one CTA an SM over all groups
+  k_ptc_wgrad<CI, CO><<<dim3(gx, WgradCfg<CI>::groups), WgradCfg<CI>::threads, sm, L.stream>>>(a, ntiles);
   YG_LAUNCHED();
   return gx;
 }
@@ -684,7 +703,7 @@ PtcArgs base_args(Ptc &n) {
   a.g = n.L->g;
   a.U = n.L->links.as<double2>();
   a.err = n.err.as<int>();
-  a.V = (int)n.L->V;
+  a.V = a.nout = (int)n.L->V;
   return a;
 }
 
@@ -762,20 +781,31 @@ void ptc_get_weights(Ptc &n, int l, double *w) {
   std::memcpy(w, n.W[l].data(), sizeof(double) * n.W[l].size());
 }
 
-// one layer on activation planes (adjoint: the input-gradient layer, Co -> Ci channels)
-void ptc_layer(Ptc &n, int l, int adjoint, const float *in, float *out) {
-  if (l < 0 || l >= n.nl) throw Error(YG_ERR_ARG, "layer index");
+// The network maps even-site vectors to even-site vectors: the first layer's input (and the last
+// layer's output gradient) vanishes on the odd sites, of which the last layer's output is not wanted.
+// Zeros that are known are neither gathered nor multiplied (with even-odd site order).
+static void layer(Ptc &n, int l, int adjoint, const float *in, float *out, bool in_even, bool out_even) {
   PtcArgs a = base_args(n);
   a.in = in;
   a.out = out;
+  a.in_even = in_even && n.L->p.eo;
+  if (out_even && n.L->p.eo) a.nout = (int)n.L->Vh;
   const int ci = adjoint ? n.ch[l + 1] : n.ch[l], co = adjoint ? n.ch[l] : n.ch[l + 1];
   a.A = (adjoint ? n.Aa[l] : n.Af[l]).as<__nv_bfloat16>();
   YG_PTC_DISPATCH(ci, co, run_layer<CI, CO>(*n.L, a));
 }
 
-// forward through all layers from act[0]; act[l] keeps every layer's input
+// one layer on activation planes (adjoint: the input-gradient layer, Co -> Ci channels)
+void ptc_layer(Ptc &n, int l, int adjoint, const float *in, float *out) {
+  if (l < 0 || l >= n.nl) throw Error(YG_ERR_ARG, "layer index");
+  layer(n, l, adjoint, in, out, false, false);
+}
+
+// forward through all layers from act[0]; act[l] keeps every layer's input, act[nl] the output on the
+// even sites
 static void forward(Ptc &n) {
-  for (int l = 0; l < n.nl; l++) ptc_layer(n, l, 0, n.act[l].as<float>(), n.act[l + 1].as<float>());
+  for (int l = 0; l < n.nl; l++)
+    layer(n, l, 0, n.act[l].as<float>(), n.act[l + 1].as<float>(), l == 0, l == n.nl - 1);
 }
 
 void ptc_apply(Ptc &n, double *dst, const double *src) {
@@ -814,6 +844,8 @@ static void wgrad(Ptc &n, int l, const float *gin, std::vector<double> &grads) {
   PtcArgs a = base_args(n);
   a.in = n.act[l].as<float>();
   a.gin = gin;
+  a.in_even = l == 0 && L.p.eo;
+  if (l == n.nl - 1 && L.p.eo) a.nout = (int)L.Vh;      // the loss sees the even sites
   a.part = n.part.as<float>();
   int gx = 0;
   YG_PTC_DISPATCH(ci, co, gx = run_wgrad<CI, CO>(L, a, sms));
@@ -863,7 +895,7 @@ void ptc_backward(Ptc &n, const double *src, const double *gout, double *grads_o
   for (int l = n.nl - 1; l >= 0; l--) {
     wgrad(n, l, gcur, grads[l]);
     if (l > 0) {
-      ptc_layer(n, l, 1, gcur, gnext);
+      layer(n, l, 1, gcur, gnext, l == n.nl - 1, false);
       std::swap(gcur, gnext);
     }
   }
@@ -907,7 +939,7 @@ double ptc_gradient(Ptc &n, int npairs, double *const *r, double *const *e, doub
     for (int l = n.nl - 1; l >= 0; l--) {
       wgrad(n, l, gcur, grads[l]);
       if (l > 0) {
-        ptc_layer(n, l, 1, gcur, gnext);
+        layer(n, l, 1, gcur, gnext, l == n.nl - 1, false);
         std::swap(gcur, gnext);
       }
     }
