@@ -328,13 +328,9 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
     double *t = l.scratch_field(2), *o = l.scratch_field(1);
     long lo, cnt;
     l.view_range(YG_VIEW_DEFAULT, lo, cnt);
-    blas_copy(l, p, xs[i]);
-    apply_op(l, YG_OP_HPHI_SQ, mass, q, p);    // also builds the clover inverse for this mass
-    blas_copy(l, r, bs[i]);
-    blas_axpby(l, r, make_double2(1, 0), make_double2(-1, 0), q, lo, cnt);
-    blas_copy(l, p, r);
+    const double rr = true_residual(l, mass, r, q, p, xs[i], bs[i], lo, cnt);   // also builds the clover inverse
+    blas_copy_range(l, p, r, lo, cnt);
     const double norm = blas_sqnorm(l, bs[i], lo, cnt);
-    const double rr = blas_sqnorm(l, r, lo, cnt);
     BLat &b = h[i];
     b.g = l.g;
     b.U = l.links.as<double2>();

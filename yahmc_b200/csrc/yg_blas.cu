@@ -157,6 +157,33 @@ void blas_copy(Lattice &L, double *dst, const double *src) {
   YG_CUDA(cudaMemcpyAsync(dst, src, L.field_bytes(), cudaMemcpyDeviceToDevice, L.stream));
 }
 
+void blas_copy_range(Lattice &L, double *dst, const double *src, long lo, long n) {
+  YG_CUDA(cudaMemcpyAsync((double2 *)dst + woff(L, lo), (const double2 *)src + woff(L, lo), sizeof(double2) * wcnt(L, n),
+                          cudaMemcpyDeviceToDevice, L.stream));
+}
+
+// r = b - q ; partial |r|^2
+__global__ void __launch_bounds__(256) k_residual(double2 *partial, double2 *r, const double2 *b, const double2 *q,
+                                                  long n) {
+  double2 acc = make_double2(0, 0);
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    const double2 v = csub(b[i], q[i]);
+    r[i] = v;
+    acc.x = fma(v.x, v.x, fma(v.y, v.y, acc.x));
+  }
+  acc = block_sum2(acc);
+  if (threadIdx.x == 0) partial[blockIdx.x] = acc;
+}
+
+double blas_residual(Lattice &L, double *r, const double *b, const double *q, long lo, long n) {
+  const long cnt = wcnt(L, n), o = woff(L, lo);
+  const int grid = red_grid(L, cnt);
+  k_residual<<<grid, 256, 0, L.stream>>>(L.red_partial.as<double2>(), (double2 *)r + o, (const double2 *)b + o,
+                                         (const double2 *)q + o, cnt);
+  YG_LAUNCHED();
+  return reduce_partials(L, grid).x;
+}
+
 void blas_zero(Lattice &L, double *f, long lo, long n) {
   YG_CUDA(cudaMemsetAsync((double2 *)f + woff(L, lo), 0, sizeof(double2) * wcnt(L, n), L.stream));
 }
@@ -301,7 +328,7 @@ void f_xpay(Lattice &L, float *p, float b, const float *r, long cnt) {
   YG_LAUNCHED();
 }
 
-// ---- cg_mshift updates of all shifts in one pass each (cg.cpp:62-116)
+// ---- cg_mshift updates (cg.cpp:62-116): r += beta q with |r|^2, then all active shifts at once
 // Launch parameters carry the per-shift fields and coefficients of the active shifts.
 struct MshiftArgs {
   double2 *x[kMaxShifts];
@@ -312,9 +339,8 @@ struct MshiftArgs {
   int num;
 };
 
-// r += beta q (partial |r|^2) and x_n -= bt_n k_n for every active shift, one pass
-__global__ void __launch_bounds__(256) k_mshift_xr(double2 *partial, double2 *r, const double2 *q, double beta,
-                                                   MshiftArgs a, long n) {
+// r += beta q ; partial |r|^2
+__global__ void __launch_bounds__(256) k_mshift_r(double2 *partial, double2 *r, const double2 *q, double beta, long n) {
   double acc = 0.0;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     double2 v = r[i], w = q[i];
@@ -322,26 +348,33 @@ __global__ void __launch_bounds__(256) k_mshift_xr(double2 *partial, double2 *r,
     v.y = fma(beta, w.y, v.y);
     r[i] = v;
     acc = fma(v.x, v.x, fma(v.y, v.y, acc));
-    for (int s = 0; s < a.num; s++) {
-      double2 xv = a.x[s][i], kv = a.k[s][i];
-      xv.x = fma(-a.c_x[s], kv.x, xv.x);
-      xv.y = fma(-a.c_x[s], kv.y, xv.y);
-      a.x[s][i] = xv;
-    }
   }
   double2 t = block_sum2(make_double2(acc, 0.0));
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
 }
 
-// k_n = at_n k_n + c3_n r for every active shift, and p = alpha p + r, one pass
-__global__ void __launch_bounds__(256) k_mshift_kp(double2 *p, const double2 *r, double alpha, MshiftArgs a, long n) {
+// x_n -= bt_n k_n and k_n = at_n k_n + c3_n r for every active shift, and p = alpha p + r: the search
+// vectors are read and written once an iteration, which is what bounds the solver with many shifts
+// (with x_n updated in the pass over r, k_n was read twice: 323 + 224 us an iteration for 12 shifts on
+// 48 x 24^3, d = 3).  first != null: the k_n still equal it (the source) and are not read.  p == null
+// ends the solve: only x_n is wanted.
+template <bool FIRST>
+__global__ void __launch_bounds__(256) k_mshift_xkp(double2 *p, const double2 *r, double alpha,
+                                                    const __grid_constant__ MshiftArgs a, const double2 *first, long n) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const double2 rv = r[i];
+    const double2 f = FIRST ? first[i] : make_double2(0, 0);
+#pragma unroll 4
     for (int s = 0; s < a.num; s++) {
-      double2 kv = a.k[s][i];
-      kv.x = fma(a.c_kr[s], rv.x, a.c_kk[s] * kv.x);
-      kv.y = fma(a.c_kr[s], rv.y, a.c_kk[s] * kv.y);
-      a.k[s][i] = kv;
+      double2 kv = FIRST ? f : a.k[s][i], xv = a.x[s][i];
+      xv.x = fma(-a.c_x[s], kv.x, xv.x);
+      xv.y = fma(-a.c_x[s], kv.y, xv.y);
+      a.x[s][i] = xv;
+      if (p) {
+        kv.x = fma(a.c_kr[s], rv.x, a.c_kk[s] * kv.x);
+        kv.y = fma(a.c_kr[s], rv.y, a.c_kk[s] * kv.y);
+        a.k[s][i] = kv;
+      }
     }
     if (p) {
       double2 pv = p[i];
@@ -350,39 +383,69 @@ __global__ void __launch_bounds__(256) k_mshift_kp(double2 *p, const double2 *r,
   }
 }
 
-static MshiftArgs mshift_args(const Lattice &L, int num, double *const *x, double *const *k, const double *c1,
-                              const double *c2, const double *c3, long lo) {
-  if (num < 0 || num > kMaxShifts) throw Error(YG_ERR_ARG, "too many shifts");
-  MshiftArgs a{};
-  a.num = num;
-  const long o = woff(L, lo);
-  for (int s = 0; s < num; s++) {
-    a.x[s] = x ? (double2 *)x[s] + o : nullptr;
-    a.k[s] = (double2 *)k[s] + o;
-    a.c_x[s] = c1 ? c1[s] : 0.0;
-    a.c_kk[s] = c2 ? c2[s] : 0.0;
-    a.c_kr[s] = c3 ? c3[s] : 0.0;
-  }
-  return a;
-}
-
-double blas_mshift_xr(Lattice &L, double *r, const double *q, double beta, int num, double *const *x,
-                      double *const *k, const double *bt, long lo, long n) {
-  long cnt = wcnt(L, n);
-  int grid = red_grid(L, cnt);
-  MshiftArgs a = mshift_args(L, num, x, k, bt, nullptr, nullptr, lo);
-  k_mshift_xr<<<grid, 256, 0, L.stream>>>(L.red_partial.as<double2>(), (double2 *)r + woff(L, lo),
-                                           (const double2 *)q + woff(L, lo), beta, a, cnt);
+double blas_mshift_r(Lattice &L, double *r, const double *q, double beta, long lo, long n) {
+  const long cnt = wcnt(L, n);
+  const int grid = red_grid(L, cnt);
+  k_mshift_r<<<grid, 256, 0, L.stream>>>(L.red_partial.as<double2>(), (double2 *)r + woff(L, lo),
+                                         (const double2 *)q + woff(L, lo), beta, cnt);
   YG_LAUNCHED();
   return reduce_partials(L, grid).x;
 }
 
-void blas_mshift_kp(Lattice &L, double *p, const double *r, double alpha, int num, double *const *k,
-                    const double *at, const double *c3, long lo, long n) {
-  long cnt = wcnt(L, n);
-  MshiftArgs a = mshift_args(L, num, nullptr, k, nullptr, at, c3, lo);
-  k_mshift_kp<<<stream_grid(cnt), 256, 0, L.stream>>>(p ? (double2 *)p + woff(L, lo) : nullptr,
-                                                       (const double2 *)r + woff(L, lo), alpha, a, cnt);
+void blas_mshift_xkp(Lattice &L, double *p, const double *r, double alpha, int num, double *const *x, double *const *k,
+                     const double *bt, const double *at, const double *c3, const double *first, long lo, long n) {
+  if (num < 0 || num > kMaxShifts) throw Error(YG_ERR_ARG, "too many shifts");
+  MshiftArgs a{};
+  a.num = num;
+  const long o = woff(L, lo), cnt = wcnt(L, n);
+  for (int s = 0; s < num; s++) {
+    a.x[s] = (double2 *)x[s] + o;
+    a.k[s] = (double2 *)k[s] + o;
+    a.c_x[s] = bt[s];
+    a.c_kk[s] = at[s];
+    a.c_kr[s] = c3[s];
+  }
+  double2 *po = p ? (double2 *)p + o : nullptr;
+  if (first)
+    k_mshift_xkp<true><<<stream_grid(cnt), 256, 0, L.stream>>>(po, (const double2 *)r + o, alpha, a,
+                                                                (const double2 *)first + o, cnt);
+  else
+    k_mshift_xkp<false><<<stream_grid(cnt), 256, 0, L.stream>>>(po, (const double2 *)r + o, alpha, a, nullptr, cnt);
+  YG_LAUNCHED();
+}
+
+// x = a0 b + sum_n c_n y_n in one pass
+struct CombineArgs {
+  const double2 *y[kMaxShifts];
+  double c[kMaxShifts];
+  int num;
+};
+
+__global__ void __launch_bounds__(256) k_combine(double2 *x, const double2 *b, double a0,
+                                                 const __grid_constant__ CombineArgs a, long n) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    double2 v = cscale(b[i], a0);
+#pragma unroll 4
+    for (int s = 0; s < a.num; s++) {
+      const double2 y = a.y[s][i];
+      v.x = fma(a.c[s], y.x, v.x);
+      v.y = fma(a.c[s], y.y, v.y);
+    }
+    x[i] = v;
+  }
+}
+
+void blas_combine(Lattice &L, double *x, const double *b, double a0, int num, double *const *y, const double *c, long lo,
+                  long n) {
+  if (num < 0 || num > kMaxShifts) throw Error(YG_ERR_ARG, "too many terms");
+  CombineArgs a{};
+  a.num = num;
+  const long o = woff(L, lo), cnt = wcnt(L, n);
+  for (int s = 0; s < num; s++) {
+    a.y[s] = (const double2 *)y[s] + o;
+    a.c[s] = c[s];
+  }
+  k_combine<<<stream_grid(cnt), 256, 0, L.stream>>>((double2 *)x + o, (const double2 *)b + o, a0, a, cnt);
   YG_LAUNCHED();
 }
 

@@ -120,11 +120,12 @@ void schur_step2(Lattice &L, double mass, double *dst, const double *tmp, const 
 }
 
 // Dphi with the reference's side effects (dirac.cpp:738-765)
-static void dphi_impl(Lattice &L, double mass, double *dst, double *src, bool g5) {
+static void dphi_impl(Lattice &L, double mass, double *dst, double *src, bool g5, bool mark = true) {
   if (L.p.eo) {
     if (L.p.clover) {
       double *tmp = L.scratch_field(1);
-      schur_step1(L, mass, tmp, src, src);        // src_o = 1/2 H src_e (in place, as the reference)
+      // src_o = 1/2 H src_e (in place, as the reference): a field's worth of writes in the step's 13
+      schur_step1(L, mass, tmp, src, mark ? src : nullptr);
       schur_step2(L, mass, dst, tmp, src, g5);
     } else {
       auto a = base_args<double>(L);
@@ -161,19 +162,33 @@ static void dphi_impl(Lattice &L, double mass, double *dst, double *src, bool g5
 void dphi(Lattice &L, double mass, double *dst, double *src) { dphi_impl(L, mass, dst, src, false); }
 void hphi(Lattice &L, double mass, double *dst, double *src) { dphi_impl(L, mass, dst, src, true); }
 
-void hphi_sq(Lattice &L, double mass, double *dst, double *src) {
+static void hphi_sq_impl(Lattice &L, double mass, double *dst, double *src, bool mark) {
   double *tmp = L.scratch_field(2);
-  hphi(L, mass, tmp, src);
-  hphi(L, mass, dst, tmp);
+  dphi_impl(L, mass, tmp, src, true, mark);
+  dphi_impl(L, mass, dst, tmp, true, false);
 }
 
-void apply_op(Lattice &L, int op, double mass, double *dst, double *src) {
+void hphi_sq(Lattice &L, double mass, double *dst, double *src) { hphi_sq_impl(L, mass, dst, src, true); }
+
+void apply_op(Lattice &L, int op, double mass, double *dst, double *src, bool mark) {
   switch (op) {
-    case YG_OP_DPHI: dphi(L, mass, dst, src); return;
-    case YG_OP_HPHI: hphi(L, mass, dst, src); return;
-    case YG_OP_HPHI_SQ: hphi_sq(L, mass, dst, src); return;
+    case YG_OP_DPHI: dphi_impl(L, mass, dst, src, false, mark); return;
+    case YG_OP_HPHI: dphi_impl(L, mass, dst, src, true, mark); return;
+    case YG_OP_HPHI_SQ: hphi_sq_impl(L, mass, dst, src, mark); return;
   }
   throw Error(YG_ERR_ARG, "invalid operator id");
+}
+
+double true_residual(Lattice &L, double mass, double *r, double *Ax, double *tmp, const double *x, const double *b,
+                     long lo, long n) {
+  // without a clover term the operator works in the source's odd half, and open / SF boundaries are
+  // applied to the source: those get a copy
+  if (!L.p.clover || !L.p.eo || has_spinor_bcs(L)) {
+    blas_copy_range(L, tmp, x, lo, n);
+    x = tmp;
+  }
+  apply_op(L, YG_OP_HPHI_SQ, mass, Ax, const_cast<double *>(x), false);
+  return blas_residual(L, r, b, Ax, lo, n);
 }
 
 // ------------------------------------------------------------------ FP32 inner operator

@@ -160,7 +160,13 @@ void schur_step2(Lattice &L, double mass, double *dst, const double *tmp, const 
 void dphi(Lattice &L, double mass, double *dst, double *src);
 void hphi(Lattice &L, double mass, double *dst, double *src);
 void hphi_sq(Lattice &L, double mass, double *dst, double *src);
-void apply_op(Lattice &L, int op, double mass, double *dst, double *src);
+// mark = false: the reference's writes into the source (its odd half, boundary slices) are not wanted,
+// because it is the caller's own; then the source stays as it is, except that open and SF boundaries
+// are applied to it
+void apply_op(Lattice &L, int op, double mass, double *dst, double *src, bool mark = true);
+// r = b - Hphi_sq x in FP64, returns |r|^2; Ax and tmp are scratch, x stays as it is
+double true_residual(Lattice &L, double mass, double *r, double *Ax, double *tmp, const double *x, const double *b,
+                     long lo, long n);
 void hphi_float(Lattice &L, double mass, float2 *dst, float2 *src, float2 *tmp);
 
 // ---- yg_blas.cu: BLAS-1 (linalg.cpp) over [lo, lo+n) sites
@@ -171,6 +177,9 @@ double blas_product_re(Lattice &L, const double *a, const double *b, long lo, lo
 void blas_axpby(Lattice &L, double *lhs, double2 alpha, double2 beta, const double *rhs, long lo, long n);
 void blas_g5(Lattice &L, double *f, long lo, long n);
 void blas_copy(Lattice &L, double *dst, const double *src);
+void blas_copy_range(Lattice &L, double *dst, const double *src, long lo, long n);
+// r = b - q, returns |r|^2
+double blas_residual(Lattice &L, double *r, const double *b, const double *q, long lo, long n);
 void blas_zero(Lattice &L, double *f, long lo, long n);
 // fused CG update: x += a p ; r -= a q ; return |r|^2
 double blas_cg_update(Lattice &L, double *x, double *r, const double *p, const double *q, double a, long lo, long n);
@@ -178,12 +187,14 @@ double sum_device(Lattice &L, const double *v, long n);
 // sum the first `grid` double2 partials in L.red_partial (deterministic), to the host
 double2 reduce_partials(Lattice &L, int grid);
 constexpr int kMaxShifts = 50;          // MAX of cg.cpp:5
-// cg_mshift passes over all active shifts at once: r += beta q, x_n -= bt_n k_n (returns
-// |r|^2); and k_n = at_n k_n + c3_n r, p = alpha p + r (p may be null)
-double blas_mshift_xr(Lattice &L, double *r, const double *q, double beta, int num, double *const *x,
-                      double *const *k, const double *bt, long lo, long n);
-void blas_mshift_kp(Lattice &L, double *p, const double *r, double alpha, int num, double *const *k,
-                    const double *at, const double *c3, long lo, long n);
+// cg_mshift: r += beta q, returns |r|^2; then over all active shifts x_n -= bt_n k_n, k_n = at_n k_n +
+// c3_n r (k_n = first before the first update when first is given), p = alpha p + r (p null: x_n only)
+double blas_mshift_r(Lattice &L, double *r, const double *q, double beta, long lo, long n);
+void blas_mshift_xkp(Lattice &L, double *p, const double *r, double alpha, int num, double *const *x, double *const *k,
+                     const double *bt, const double *at, const double *c3, const double *first, long lo, long n);
+// x = a0 b + sum_n c_n y_n
+void blas_combine(Lattice &L, double *x, const double *b, double a0, int num, double *const *y, const double *c, long lo,
+                  long n);
 // FP32 helpers of the mixed-precision solver (counts in complex words)
 void f_from_d(Lattice &L, float *dst, const double *src, long cnt);
 void d_add_f(Lattice &L, double *dst, const float *src, long cnt);

@@ -542,11 +542,7 @@ int cg_mixed_mrhs(Lattice &L, const yg_inv_par &par, int nrhs, double *const *xs
   double *r64 = L.scratch_field(3), *Ax = L.scratch_field(4), *xd = L.scratch_field(5);
 
   auto residual = [&](int i) {      // r64 = b_i - A x_i in FP64, returns |r|^2
-    blas_copy(L, xd, xs[i]);
-    apply_op(L, YG_OP_HPHI_SQ, mass[i], Ax, xd);
-    blas_copy(L, r64, bs[i]);
-    blas_axpby(L, r64, make_double2(1, 0), make_double2(-1, 0), Ax, lo, n);
-    return blas_sqnorm(L, r64, lo, n);
+    return true_residual(L, mass[i], r64, Ax, xd, xs[i], bs[i], lo, n);
   };
   auto set_scalar = [&](int idx, double v) {
     k_m_set<<<1, 1, 0, L.stream>>>(scal, idx, v);

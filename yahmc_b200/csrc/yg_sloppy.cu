@@ -893,11 +893,7 @@ int cg_mixed_sloppy(Lattice &L, const yg_inv_par &par, int prec, int reals, int 
   set_scalar(L, S_ITER, 0.0);       // the device's count of finished inner iterations
 
   auto residual = [&]() {           // r = b - A x in FP64, returns |r|^2
-    blas_copy(L, xd, x);
-    apply_op(L, YG_OP_HPHI_SQ, par.mass, Ax, xd);
-    blas_copy(L, r, b);
-    blas_axpby(L, r, make_double2(1, 0), make_double2(-1, 0), Ax, lo, n);
-    return blas_sqnorm(L, r, lo, n);
+    return true_residual(L, par.mass, r, Ax, xd, x, b, lo, n);
   };
 
   double norm = blas_sqnorm(L, b, lo, n);

@@ -60,18 +60,16 @@ void check_finite(double v, const char *what) {
 static int cg_launches(Lattice &L, const yg_inv_par &par, double *x, double *b, int *iters) {
   Ctx c(L);
   double *r = L.scratch_field(3), *p = L.scratch_field(4), *q = L.scratch_field(5);
-  c.copy(p, x);
-  apply_op(L, par.op, par.mass, q, p);
-  c.copy(r, b);
-  c.axpby(r, {1, 0}, {-1, 0}, q);
-  c.copy(p, r);
+  blas_copy_range(L, p, x, c.lo, c.n);
+  apply_op(L, par.op, par.mass, q, p, false);
   double norm = c.sqnorm(b);
-  double rr = c.sqnorm(r);
+  double rr = blas_residual(L, r, b, q, c.lo, c.n);
+  blas_copy_range(L, p, r, c.lo, c.n);
   int it = (rr < norm * par.prec) ? -1 : 0;
   int status = YG_OK;
   while (++it) {
     if (par.maxiter > 0 && it > par.maxiter) { it--; status = YG_MAXITER; break; }
-    apply_op(L, par.op, par.mass, q, p);
+    apply_op(L, par.op, par.mass, q, p, false);
     double atmp = rr;                       // = spinor_sqnorm(r) of cg.cpp:176, unchanged since
     double pq = c.prod_re(p, q);
     check_finite(pq, "cg");
@@ -161,12 +159,9 @@ int cg_mshift(Lattice &L, const yg_inv_par &par, int num, const double *shift, d
   double *r = L.scratch_field(3), *p = L.scratch_field(4), *q = L.scratch_field(5);
   std::vector<double *> k(num);
   for (int n = 0; n < num; n++) k[n] = L.scratch_field(10 + n);
-  c.copy(r, b);
-  c.copy(p, b);
-  for (int n = 0; n < num; n++) {
-    blas_zero(L, xs[n], 0, L.V);
-    c.copy(k[n], b);
-  }
+  blas_copy_range(L, r, b, c.lo, c.n);
+  blas_copy_range(L, p, b, c.lo, c.n);
+  for (int n = 0; n < num; n++) blas_zero(L, xs[n], 0, L.V);      // k_n = b: read from b in the first iteration
   std::vector<double> c1(num, 1.0), c2(num, 1.0), c3(num, 0.0);
   std::vector<int> flag(num, 0);
   double beta = 1, alpha = 0, btmp = 0;
@@ -174,12 +169,12 @@ int cg_mshift(Lattice &L, const yg_inv_par &par, int num, const double *shift, d
   double atmp = c.sqnorm(r);
   int it = 0;
   int status = YG_OK;
-  // the per-shift x and k updates of one iteration run as one pass each over all active
-  // shifts (blas_mshift_xr / _kp); scalars follow cg.cpp:62-116 in the same order
+  // the per-shift x and k updates of one iteration run as one pass over all active shifts
+  // (blas_mshift_xkp); scalars follow cg.cpp:62-116 in the same order
   std::vector<double *> ax(num), ak(num);
   std::vector<double> abt(num), aat(num), ac3(num);
   while (++it) {
-    apply_op(L, par.op, par.mass, q, p);
+    apply_op(L, par.op, par.mass, q, p, false);
     double pq = c.prod_re(p, q);
     check_finite(pq, "cg_mshift");
     double beta_old = beta;
@@ -194,7 +189,7 @@ int cg_mshift(Lattice &L, const yg_inv_par &par, int num, const double *shift, d
       abt[na] = beta * (c3[n] / c2[n]);
       na++;
     }
-    btmp = blas_mshift_xr(L, r, q, beta, na, ax.data(), ak.data(), abt.data(), c.lo, c.n);
+    btmp = blas_mshift_r(L, r, q, beta, c.lo, c.n);
     alpha = btmp / atmp;
     int notconverged = 0;
     na = 0;
@@ -209,10 +204,11 @@ int cg_mshift(Lattice &L, const yg_inv_par &par, int num, const double *shift, d
       c1[n] = c2[n];
       c2[n] = c3[n];
     }
-    // k_n = at k_n + c3 r for the shifts active in this iteration; p = alpha p + r is only
-    // needed when the loop goes on
+    // x_n -= bt k_n for the shifts active in this iteration; k_n = at k_n + c3 r and p = alpha p + r
+    // are only needed when the loop goes on
     bool more = notconverged > 0 && !(par.maxiter > 0 && it >= par.maxiter);
-    blas_mshift_kp(L, more ? p : nullptr, r, alpha, na, ak.data(), aat.data(), ac3.data(), c.lo, c.n);
+    blas_mshift_xkp(L, more ? p : nullptr, r, alpha, na, ax.data(), ak.data(), abt.data(), aat.data(), ac3.data(),
+                    it == 1 ? b : nullptr, c.lo, c.n);
     if (notconverged == 0) break;
     if (par.maxiter > 0 && it >= par.maxiter) { status = YG_MAXITER; break; }
     atmp = btmp;
@@ -239,11 +235,11 @@ int bicgstab(Lattice &L, const yg_inv_par &par, double *x, double *b, int *iters
   int status = YG_OK;
   while (++it) {
     if (par.maxiter > 0 && it > par.maxiter) { it--; status = YG_MAXITER; break; }
-    apply_op(L, par.op, par.mass, v, p);
+    apply_op(L, par.op, par.mass, v, p, false);
     cx alpha = cdiv(rho0, c.prod(v, r0));
     check_finite(alpha.re, "bicgstab");
     c.axpby(r, {1, 0}, {-alpha.re, -alpha.im}, v);
-    apply_op(L, par.op, par.mass, t, r);
+    apply_op(L, par.op, par.mass, t, r, false);
     cx omega = c.prod(r, t);
     double tt = c.sqnorm(t);
     omega = {omega.re / tt, omega.im / tt};
@@ -286,7 +282,7 @@ int minres(Lattice &L, const yg_inv_par &par, double *x, double *b, int *iters) 
   while (++it) {
     if (par.maxiter > 0 && it > par.maxiter) { it--; status = YG_MAXITER; break; }
     c.axpby(v1, {1.0 / beta0, 0}, {0, 0}, nullptr);
-    apply_op(L, par.op, par.mass, tmp, v1);
+    apply_op(L, par.op, par.mass, tmp, v1, false);
     double alpha = c.prod_re(v1, tmp);
     check_finite(alpha, "minres");
     c.axpby(tmp, {1, 0}, {-alpha, 0}, v1);
@@ -354,8 +350,7 @@ int rational_calc(Lattice &L, const yg_inv_par &par, double a0, int order, const
   int st = cg_mshift(L, par, order, poles, outs.data(), b, iters);
   long lo, n;
   L.view_range(YG_VIEW_DEFAULT, lo, n);
-  blas_axpby(L, x, make_double2(0, 0), make_double2(a0, 0), b, lo, n);
-  for (int i = 0; i < order; i++) blas_axpby(L, x, make_double2(1, 0), make_double2(residues[i], 0), outs[i], lo, n);
+  blas_combine(L, x, b, a0, order, outs.data(), residues, lo, n);
   return st;
 }
 
@@ -385,11 +380,7 @@ int cg_mixed(Lattice &L, const yg_inv_par &par, double *x, double *b, yg_solve_s
 
   const double delta = 0.1;
   double norm = c.sqnorm(b);
-  c.copy(xd, x);
-  apply_op(L, YG_OP_HPHI_SQ, par.mass, Ax, xd);
-  c.copy(r, b);
-  c.axpby(r, {1, 0}, {-1, 0}, Ax);
-  double rr = c.sqnorm(r);
+  double rr = true_residual(L, par.mass, r, Ax, xd, x, b, c.lo, c.n);
   double target = norm * par.prec;
   int it = 0, updates = 0, status = YG_OK;
   double best = rr;
@@ -424,11 +415,7 @@ int cg_mixed(Lattice &L, const yg_inv_par &par, double *x, double *b, yg_solve_s
         // fold the FP32 increment into x and recompute the true residual in FP64
         d_add_f(L, x, fx, cnt);
         YG_CUDA(cudaMemsetAsync(fx, 0, sizeof(float2) * cnt, L.stream));
-        c.copy(xd, x);
-        apply_op(L, YG_OP_HPHI_SQ, par.mass, Ax, xd);
-        c.copy(r, b);
-        c.axpby(r, {1, 0}, {-1, 0}, Ax);
-        double rr_true = c.sqnorm(r);
+        double rr_true = true_residual(L, par.mass, r, Ax, xd, x, b, c.lo, c.n);
         updates++;
         if (rr_true < target) { rr = rr_true; break; }
         if (rr_true < best) c.copy(xbest, x);
@@ -463,11 +450,7 @@ int cg_mixed(Lattice &L, const yg_inv_par &par, double *x, double *b, yg_solve_s
       int it64 = 0;
       status = cg(L, p64, x, b, &it64);
       it += it64;
-      c.copy(xd, x);
-      apply_op(L, YG_OP_HPHI_SQ, par.mass, Ax, xd);
-      c.copy(r, b);
-      c.axpby(r, {1, 0}, {-1, 0}, Ax);
-      rr = c.sqnorm(r);
+      rr = true_residual(L, par.mass, r, Ax, xd, x, b, c.lo, c.n);
       if (status != YG_OK || rr < target) break;
     }
     if (status == YG_OK && rr >= target) status = YG_STALL;
