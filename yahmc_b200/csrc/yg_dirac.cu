@@ -43,6 +43,7 @@ static HopArgs<R> base_args(const Lattice &L) {
   HopArgs<R> a{};
   a.g = L.g;
   a.cfm1 = (R)(L.p.cf - 1.0);
+  if constexpr (sizeof(R) == sizeof(double)) a.Ur = L.links_r.as<double>();
   return a;
 }
 

@@ -15,6 +15,7 @@
 //  mixed-precision solver); storage is cplx<R>.
 #pragma once
 
+#include <type_traits>
 #include "yg_kernels.h"
 
 namespace yg {
@@ -45,17 +46,35 @@ __device__ __forceinline__ void store_spinor(cplx<R> *f, const cplx<R> (&s)[4][D
   }
 }
 
+// acc += u h for a real link entry u
+template <typename T, typename R>
+__device__ __forceinline__ void rfma(T &acc, R u, T h) {
+  acc.x = fma(u, h.x, acc.x);
+  acc.y = fma(u, h.y, acc.y);
+}
+
+// The links a hop reads: complex, or (adjoint representations, FP64) the real copy, half the bytes.
+// The product with an imaginary part of zero is the same number.
+template <typename R, bool REAL> struct LinkPtr { using t = const cplx<R> *; };
+template <typename R> struct LinkPtr<R, true> { using t = const R *; };
+template <bool REAL, typename R>
+__device__ __forceinline__ typename LinkPtr<R, REAL>::t hop_links(const HopArgs<R> &a) {
+  if constexpr (REAL) return a.Ur;
+  else return a.U;
+}
+
 // chi = U h (DAG=false) or U^dag h (DAG=true), U = link (id, mu)
-template <int D, typename R, bool DAG>
-__device__ __forceinline__ void link_mul(cplx<R> (&chi)[2][D], const cplx<R> (&h)[2][D], const cplx<R> *U,
-                                         const Geom &g, int id, int mu) {
+template <int D, typename R, bool DAG, typename LP>
+__device__ __forceinline__ void link_mul(cplx<R> (&chi)[2][D], const cplx<R> (&h)[2][D], LP U, const Geom &g, int id,
+                                         int mu) {
   YG_UNROLL_D
   for (int i = 0; i < D; i++) {
     cplx<R> s0 = mk<R>(0, 0), s1 = mk<R>(0, 0);
     YG_UNROLL_D
     for (int j = 0; j < D; j++) {
-      cplx<R> u = ld(U, fidx(g, id, mu * D * D + (DAG ? j * D + i : i * D + j), 4 * D * D));
-      if (DAG) { cfmac(s0, u, h[0][j]); cfmac(s1, u, h[1][j]); }
+      const auto u = ld(U, fidx(g, id, mu * D * D + (DAG ? j * D + i : i * D + j), 4 * D * D));
+      if constexpr (std::is_same_v<LP, const R *>) { rfma(s0, u, h[0][j]); rfma(s1, u, h[1][j]); }
+      else if (DAG) { cfmac(s0, u, h[0][j]); cfmac(s1, u, h[1][j]); }
       else { cfma(s0, u, h[0][j]); cfma(s1, u, h[1][j]); }
     }
     chi[0][i] = s0;
@@ -64,9 +83,9 @@ __device__ __forceinline__ void link_mul(cplx<R> (&chi)[2][D], const cplx<R> (&h
 }
 
 // One direction: SIG = -1 for the forward term (1-g_mu), +1 for the backward term (1+g_mu).
-template <int D, typename R, int MU, int SIG, bool NC>
-__device__ __forceinline__ void hop_dir(cplx<R> (&acc)[4][D], const cplx<R> *src, const cplx<R> *U,
-                                        const Geom &g, int nid, int lid) {
+template <int D, typename R, int MU, int SIG, bool NC, typename LP>
+__device__ __forceinline__ void hop_dir(cplx<R> (&acc)[4][D], const cplx<R> *src, LP U, const Geom &g, int nid,
+                                        int lid) {
   cplx<R> h[2][D];
   YG_UNROLL_D
   for (int c = 0; c < D; c++) {
@@ -110,9 +129,9 @@ __device__ __forceinline__ void hop_dir(cplx<R> (&acc)[4][D], const cplx<R> *src
   }
 }
 
-template <int D, typename R, bool NC>
-__device__ __forceinline__ void hop_site(cplx<R> (&acc)[4][D], const cplx<R> *src, const cplx<R> *U, const Geom &g,
-                                         int id, const int c[4]) {
+template <int D, typename R, bool NC, typename LP>
+__device__ __forceinline__ void hop_site(cplx<R> (&acc)[4][D], const cplx<R> *src, LP U, const Geom &g, int id,
+                                         const int c[4]) {
 #pragma unroll
   for (int s = 0; s < 4; s++) {
     YG_UNROLL_D
@@ -173,24 +192,33 @@ __device__ __forceinline__ void clover_add_site(cplx<R> (&acc)[4][D], const cplx
       p0[c] = ldf<NC>(src2, fidx(g, id, s0 * D + c, 4 * D));
       p1[c] = ldf<NC>(src2, fidx(g, id, s1 * D + c, 4 * D));
     }
+    // each entry is loaded once: A0 is Hermitian to the last bit, so its lower triangle serves both
+    // triangles and, negated, the lower spin; A1 serves the upper spin and, daggered, the lower one
 #pragma unroll
     for (int i = 0; i < D; i++) {
-      cplx<R> o0 = cadd(acc[s0][i], cscale(p0[i], diag)), o1 = cadd(acc[s1][i], cscale(p1[i], diag));
+      acc[s0][i] = cadd(acc[s0][i], cscale(p0[i], diag));
+      acc[s1][i] = cadd(acc[s1][i], cscale(p1[i], diag));
+    }
+#pragma unroll
+    for (int i = 0; i < D; i++)
+#pragma unroll
+      for (int j = 0; j <= i; j++) {
+        const cplx<R> e = ld(cl, fidx(g, id, m0 * D * D + i * D + j, 4 * D * D)), ne = mk<R>(-e.x, -e.y);
+        cfma(acc[s0][i], e, p0[j]);
+        cfma(acc[s1][i], ne, p1[j]);
+        if (j < i) {
+          cfmac(acc[s0][j], e, p0[i]);
+          cfmac(acc[s1][j], ne, p1[i]);
+        }
+      }
+#pragma unroll
+    for (int i = 0; i < D; i++)
 #pragma unroll
       for (int j = 0; j < D; j++) {
-        // A0 and A2 are Hermitian to the last bit: only their lower triangles are read
-        cplx<R> a0 = ld(cl, fidx(g, id, m0 * D * D + (i >= j ? i * D + j : j * D + i), 4 * D * D));
-        if (i < j) a0.y = -a0.y;
-        cplx<R> a1 = ld(cl, fidx(g, id, m1 * D * D + i * D + j, 4 * D * D));
-        cplx<R> a1t = ld(cl, fidx(g, id, m1 * D * D + j * D + i, 4 * D * D));
-        cfma(o0, a0, p0[j]);
-        cfma(o0, a1, p1[j]);
-        cfmac(o1, a1t, p0[j]);
-        o1 = csub(o1, cmul(a0, p1[j]));
+        const cplx<R> w = ld(cl, fidx(g, id, m1 * D * D + i * D + j, 4 * D * D));
+        cfma(acc[s0][i], w, p1[j]);
+        cfmac(acc[s1][j], w, p0[i]);
       }
-      acc[s0][i] = o0;
-      acc[s1][i] = o1;
-    }
   }
 }
 
@@ -292,14 +320,14 @@ __device__ __forceinline__ void cpk_site(cplx<R> (&out)[4][D], const cplx<R> (&s
 }
 
 // One output site of the launch's range: its four spins in acc, for the caller to store
-template <int D, typename R, int EPI, bool NC>
+template <int D, typename R, int EPI, bool NC, bool REAL = false>
 __device__ __forceinline__ void hop_values(const HopArgs<R> &a, int t, cplx<R> (&acc)[4][D]) {
   const Geom &g = a.g;
   int id = a.lo + t;
   int c[4];
   coords_of(g, id, c);
   bool bnd = spinor_zeroed(g, c[0]);
-  hop_site<D, R, NC>(acc, a.src, a.U, g, id, c);
+  hop_site<D, R, NC>(acc, a.src, hop_links<REAL>(a), g, id, c);
 #pragma unroll
   for (int s = 0; s < 4; s++) {
     YG_UNROLL_D
@@ -350,17 +378,13 @@ __device__ __forceinline__ void hop_values(const HopArgs<R> &a, int t, cplx<R> (
   }
 }
 
-template <int D, typename R, int EPI>
-__device__ __forceinline__ void hop_body(const HopArgs<R> &a, int t) {
-  cplx<R> acc[4][D];
-  hop_values<D, R, EPI, true>(a, t, acc);
-  store_spinor<D, R>(a.dst, acc, a.g, a.lo + t);
-}
-
-template <int D, typename R, int EPI>
+template <int D, typename R, int EPI, bool REAL>
 __global__ void __launch_bounds__(128) k_hop(HopArgs<R> a) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < a.n) hop_body<D, R, EPI>(a, t);
+  if (t >= a.n) return;
+  cplx<R> acc[4][D];
+  hop_values<D, R, EPI, true, REAL>(a, t, acc);
+  store_spinor<D, R>(a.dst, acc, a.g, a.lo + t);
 }
 
 // ------------------------------------------------------------------ four lanes a site
@@ -390,12 +414,12 @@ template <typename C>
 __device__ __forceinline__ C sel(bool p, C a, C b) { C c; c.x = p ? a.x : b.x; c.y = p ? a.y : b.y; return c; }
 
 // half spinor of the neighbour nid times the link lid: chi0, chi1
-template <int D, typename R, bool NC, bool DAG>
-__device__ __forceinline__ void quad_dir(cplx<R> (&chi)[2][D], const cplx<R> *src, const cplx<R> *U, const Geom &g,
-                                         int mu, bool swap, cplx<R> ph0, cplx<R> ph1, int nid, int lid) {
+template <int D, typename R, bool NC, bool DAG, typename LP>
+__device__ __forceinline__ void quad_dir(cplx<R> (&chi)[2][D], const cplx<R> *src, LP U, const Geom &g, int mu,
+                                          bool swap, cplx<R> ph0, cplx<R> ph1, int nid, int lid) {
   const int nb = nid >= g.Vh, lb = lid >= g.Vh;
   const cplx<R> *f = src + (long)nb * 4 * D * g.Vh + (nid - nb * g.Vh);
-  const cplx<R> *u = U + (long)(lb * 4 + mu) * D * D * g.Vh + (lid - lb * g.Vh);
+  const LP u = U + (long)(lb * 4 + mu) * D * D * g.Vh + (lid - lb * g.Vh);
   const long st = g.Vh;
   const long ox = (swap ? 3L * D : 2L * D) * st, oy = (swap ? 2L * D : 3L * D) * st;
   cplx<R> h[2][D];
@@ -411,8 +435,9 @@ __device__ __forceinline__ void quad_dir(cplx<R> (&chi)[2][D], const cplx<R> *sr
     cplx<R> c0 = mk<R>(0, 0), c1 = mk<R>(0, 0);
 #pragma unroll
     for (int j = 0; j < D; j++) {
-      const cplx<R> w = ld(u, (DAG ? j * D + i : i * D + j) * st);
-      if (DAG) { cfmac(c0, w, h[0][j]); cfmac(c1, w, h[1][j]); }
+      const auto w = ld(u, (DAG ? j * D + i : i * D + j) * st);
+      if constexpr (std::is_same_v<LP, const R *>) { rfma(c0, w, h[0][j]); rfma(c1, w, h[1][j]); }
+      else if (DAG) { cfmac(c0, w, h[0][j]); cfmac(c1, w, h[1][j]); }
       else { cfma(c0, w, h[0][j]); cfma(c1, w, h[1][j]); }
     }
     chi[0][i] = c0;
@@ -521,7 +546,7 @@ __device__ __forceinline__ void quad_clover_add(cplx<R> (&w)[D], const cplx<R> (
 // Spin q = threadIdx.x & 3 of output site t (clamped to the range by the caller; the four lanes of a
 // site and the other sites of the warp all take part): the result in w, `at` the index of its first
 // word (the others follow at Vh).
-template <int D, typename R, int EPI, bool NC>
+template <int D, typename R, int EPI, bool NC, bool REAL = false>
 __device__ __forceinline__ void hop_quad(const HopArgs<R> &a, int t, bool live, cplx<R> (&w)[D], long &at) {
   const Geom &g = a.g;
   const int q = threadIdx.x & 3, id = a.lo + t;
@@ -538,11 +563,11 @@ __device__ __forceinline__ void hop_quad(const HopArgs<R> &a, int t, bool live, 
 #pragma unroll
     for (int mu = 0; mu < 4; mu++)
       if (mu == q) n[mu] = n[mu] + 1 == g.dim[mu] ? 0 : n[mu] + 1;
-    quad_dir<D, R, NC, false>(cf, a.src, a.U, g, q, swap, ph0, ph1, id_of(g, n[0], n[1], n[2], n[3]), id);
+    quad_dir<D, R, NC, false>(cf, a.src, hop_links<REAL>(a), g, q, swap, ph0, ph1, id_of(g, n[0], n[1], n[2], n[3]), id);
 #pragma unroll
     for (int mu = 0; mu < 4; mu++) n[mu] = mu == q ? (c[mu] == 0 ? g.dim[mu] - 1 : c[mu] - 1) : c[mu];
     const int b = id_of(g, n[0], n[1], n[2], n[3]);
-    quad_dir<D, R, NC, true>(cb, a.src, a.U, g, q, swap, mk<R>(-ph0.x, -ph0.y), mk<R>(-ph1.x, -ph1.y), b, b);
+    quad_dir<D, R, NC, true>(cb, a.src, hop_links<REAL>(a), g, q, swap, mk<R>(-ph0.x, -ph0.y), mk<R>(-ph1.x, -ph1.y), b, b);
 #pragma unroll
     for (int k = 0; k < D; k++) {
       v[0][k] = cadd(cf[0][k], cb[0][k]);
@@ -595,13 +620,13 @@ __device__ __forceinline__ void hop_quad(const HopArgs<R> &a, int t, bool live, 
   }
 }
 
-template <int D, typename R, int EPI>
+template <int D, typename R, int EPI, bool REAL>
 __global__ void __launch_bounds__(128) k_hop_quad(HopArgs<R> a) {
   const int t = (blockIdx.x * 128 + threadIdx.x) >> 2;
   const bool live = t < a.n;
   cplx<R> w[D];
   long at;
-  hop_quad<D, R, EPI, true>(a, live ? t : a.n - 1, live, w, at);
+  hop_quad<D, R, EPI, true, REAL>(a, live ? t : a.n - 1, live, w, at);
   if (live) {
 #pragma unroll
     for (int k = 0; k < D; k++) a.dst[at + (long)k * a.g.Vh] = w[k];
@@ -656,18 +681,20 @@ __device__ __forceinline__ void row_gather(cplx<R> *sm, int slot, int i, int lan
 
 // row i of U h (forward, link of the site) or U^dag h (backward, link of the neighbour), added
 // to the four spin components
-template <int D, typename R, int MU, int SIG>
-__device__ __forceinline__ void row_apply(cplx<R> (&acc)[4], const cplx<R> *sm, int slot, int i, int lane,
-                                          const cplx<R> *U, const Geom &g, int lid) {
+template <int D, typename R, int MU, int SIG, typename LP>
+__device__ __forceinline__ void row_apply(cplx<R> (&acc)[4], const cplx<R> *sm, int slot, int i, int lane, LP U,
+                                          const Geom &g, int lid) {
   const int blk = lid >= g.Vh;
-  const cplx<R> *u = U + ((long)(blk * 4 + MU) * D * D + (SIG < 0 ? i * D : i)) * g.Vh + (lid - blk * g.Vh);
+  const LP u = U + ((long)(blk * 4 + MU) * D * D + (SIG < 0 ? i * D : i)) * g.Vh + (lid - blk * g.Vh);
   const long st = (long)(SIG < 0 ? 1 : D) * g.Vh;
   const cplx<R> *h = sm + slot * 2 * D * 32 + lane;
   cplx<R> c0 = mk<R>(0, 0), c1 = mk<R>(0, 0);
 #pragma unroll
   for (int j = 0; j < D; j++) {
-    const cplx<R> w = __ldg(u + j * st), h0 = h[j * 32], h1 = h[(D + j) * 32];
-    if (SIG < 0) { cfma(c0, w, h0); cfma(c1, w, h1); }
+    const auto w = __ldg(u + j * st);
+    const cplx<R> h0 = h[j * 32], h1 = h[(D + j) * 32];
+    if constexpr (std::is_same_v<LP, const R *>) { rfma(c0, w, h0); rfma(c1, w, h1); }
+    else if (SIG < 0) { cfma(c0, w, h0); cfma(c1, w, h1); }
     else { cfmac(c0, w, h0); cfmac(c1, w, h1); }
   }
   acc[0] = cadd(acc[0], c0);
@@ -764,9 +791,10 @@ __device__ __forceinline__ void row_clover(cplx<R> (&out)[4], const cplx<R> *x, 
 // block takes part (lanes beyond the range work on its last site).  acc receives the four spins of
 // the thread's colour, `at` the index of the first of them (the others follow at D Vh); false for a
 // lane beyond the range, whose result the caller drops.
-template <int D, typename R, int EPI>
+template <int D, typename R, int EPI, bool REAL>
 __device__ __forceinline__ bool hop_rows(const HopArgs<R> &a, int tile, cplx<R> *sm, cplx<R> (&acc)[4], long &at) {
   const Geom &g = a.g;
+  const auto U = hop_links<REAL>(a);
   const int lane = threadIdx.x & 31, i = threadIdx.x >> 5;
   const int t = tile * 32 + lane;
   const bool live = t < a.n;
@@ -792,34 +820,34 @@ __device__ __forceinline__ bool hop_rows(const HopArgs<R> &a, int tile, cplx<R> 
     row_gather<D, R, 3, -1>(sm, 6, i, lane, a.src, g, f[3]);
     row_gather<D, R, 3, +1>(sm, 7, i, lane, a.src, g, b[3]);
     __syncthreads();
-    row_apply<D, R, 0, -1>(acc, sm, 0, i, lane, a.U, g, id);
-    row_apply<D, R, 0, +1>(acc, sm, 1, i, lane, a.U, g, b[0]);
-    row_apply<D, R, 1, -1>(acc, sm, 2, i, lane, a.U, g, id);
-    row_apply<D, R, 1, +1>(acc, sm, 3, i, lane, a.U, g, b[1]);
-    row_apply<D, R, 2, -1>(acc, sm, 4, i, lane, a.U, g, id);
-    row_apply<D, R, 2, +1>(acc, sm, 5, i, lane, a.U, g, b[2]);
-    row_apply<D, R, 3, -1>(acc, sm, 6, i, lane, a.U, g, id);
-    row_apply<D, R, 3, +1>(acc, sm, 7, i, lane, a.U, g, b[3]);
+    row_apply<D, R, 0, -1>(acc, sm, 0, i, lane, U, g, id);
+    row_apply<D, R, 0, +1>(acc, sm, 1, i, lane, U, g, b[0]);
+    row_apply<D, R, 1, -1>(acc, sm, 2, i, lane, U, g, id);
+    row_apply<D, R, 1, +1>(acc, sm, 3, i, lane, U, g, b[1]);
+    row_apply<D, R, 2, -1>(acc, sm, 4, i, lane, U, g, id);
+    row_apply<D, R, 2, +1>(acc, sm, 5, i, lane, U, g, b[2]);
+    row_apply<D, R, 3, -1>(acc, sm, 6, i, lane, U, g, id);
+    row_apply<D, R, 3, +1>(acc, sm, 7, i, lane, U, g, b[3]);
   } else {
     row_gather<D, R, 0, -1>(sm, 0, i, lane, a.src, g, f[0]);
     row_gather<D, R, 0, +1>(sm, 1, i, lane, a.src, g, b[0]);
     row_gather<D, R, 1, -1>(sm, 2, i, lane, a.src, g, f[1]);
     row_gather<D, R, 1, +1>(sm, 3, i, lane, a.src, g, b[1]);
     __syncthreads();
-    row_apply<D, R, 0, -1>(acc, sm, 0, i, lane, a.U, g, id);
-    row_apply<D, R, 0, +1>(acc, sm, 1, i, lane, a.U, g, b[0]);
-    row_apply<D, R, 1, -1>(acc, sm, 2, i, lane, a.U, g, id);
-    row_apply<D, R, 1, +1>(acc, sm, 3, i, lane, a.U, g, b[1]);
+    row_apply<D, R, 0, -1>(acc, sm, 0, i, lane, U, g, id);
+    row_apply<D, R, 0, +1>(acc, sm, 1, i, lane, U, g, b[0]);
+    row_apply<D, R, 1, -1>(acc, sm, 2, i, lane, U, g, id);
+    row_apply<D, R, 1, +1>(acc, sm, 3, i, lane, U, g, b[1]);
     __syncthreads();
     row_gather<D, R, 2, -1>(sm, 0, i, lane, a.src, g, f[2]);
     row_gather<D, R, 2, +1>(sm, 1, i, lane, a.src, g, b[2]);
     row_gather<D, R, 3, -1>(sm, 2, i, lane, a.src, g, f[3]);
     row_gather<D, R, 3, +1>(sm, 3, i, lane, a.src, g, b[3]);
     __syncthreads();
-    row_apply<D, R, 2, -1>(acc, sm, 0, i, lane, a.U, g, id);
-    row_apply<D, R, 2, +1>(acc, sm, 1, i, lane, a.U, g, b[2]);
-    row_apply<D, R, 3, -1>(acc, sm, 2, i, lane, a.U, g, id);
-    row_apply<D, R, 3, +1>(acc, sm, 3, i, lane, a.U, g, b[3]);
+    row_apply<D, R, 2, -1>(acc, sm, 0, i, lane, U, g, id);
+    row_apply<D, R, 2, +1>(acc, sm, 1, i, lane, U, g, b[2]);
+    row_apply<D, R, 3, -1>(acc, sm, 2, i, lane, U, g, id);
+    row_apply<D, R, 3, +1>(acc, sm, 3, i, lane, U, g, b[3]);
   }
 #pragma unroll
   for (int s = 0; s < 4; s++) acc[s] = bnd ? mk<R>(0, 0) : cscale(acc[s], a.coeff);
@@ -870,12 +898,12 @@ __device__ __forceinline__ bool hop_rows(const HopArgs<R> &a, int tile, cplx<R> 
   return live;
 }
 
-template <int D, typename R, int EPI>
+template <int D, typename R, int EPI, bool REAL>
 __global__ void __launch_bounds__(32 * D) k_hop_rows(HopArgs<R> a) {
   extern __shared__ __align__(16) unsigned char hop_smem[];
   cplx<R> acc[4];
   long at;
-  if (hop_rows<D, R, EPI>(a, blockIdx.x, reinterpret_cast<cplx<R> *>(hop_smem), acc, at)) {
+  if (hop_rows<D, R, EPI, REAL>(a, blockIdx.x, reinterpret_cast<cplx<R> *>(hop_smem), acc, at)) {
 #pragma unroll
     for (int s = 0; s < 4; s++) a.dst[at + s * (long)D * a.g.Vh] = acc[s];
   }
@@ -1150,16 +1178,33 @@ __global__ void k_logdet(double *out, const double2 *ldl, int Vh) {
 }
 
 // ------------------------------------------------------------------ DK<D> launchers
-template <int D, typename R, int EPI>
-static void launch_hop(const HopArgs<R> &a, cudaStream_t s) {
+template <int D, typename R, int EPI, bool REAL>
+static void launch_hop_links(const HopArgs<R> &a, cudaStream_t s) {
   if constexpr (D <= 6) {
-    if (a.n <= kQuadSites) k_hop_quad<D, R, EPI><<<nblk(4L * a.n, 128), 128, 0, s>>>(a);
-    else k_hop<D, R, EPI><<<nblk(a.n, 128), 128, 0, s>>>(a);
+    if (a.n <= kQuadSites) k_hop_quad<D, R, EPI, REAL><<<nblk(4L * a.n, 128), 128, 0, s>>>(a);
+    else k_hop<D, R, EPI, REAL><<<nblk(a.n, 128), 128, 0, s>>>(a);
   } else {
     using T = RowTile<D, R>;
     if (T::smem > 48 * 1024)
-      cudaFuncSetAttribute(k_hop_rows<D, R, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem);
-    k_hop_rows<D, R, EPI><<<nblk(a.n, 32), T::threads, T::smem, s>>>(a);
+      cudaFuncSetAttribute(k_hop_rows<D, R, EPI, REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem);
+    k_hop_rows<D, R, EPI, REAL><<<nblk(a.n, 32), T::threads, T::smem, s>>>(a);
+  }
+}
+
+// d = 3, 8 and 15 are the adjoint dimensions of SU(2), SU(3) and SU(4); d = 8 and 15 are nothing else
+template <int D, typename R, int EPI>
+static void launch_hop(const HopArgs<R> &a, cudaStream_t s) {
+  constexpr bool fp64 = sizeof(R) == sizeof(double);
+  if constexpr (fp64 && (D == 8 || D == 15)) {
+    launch_hop_links<D, R, EPI, true>(a, s);
+  } else {
+    if constexpr (fp64 && D == 3) {
+      if (a.Ur) {
+        launch_hop_links<D, R, EPI, true>(a, s);
+        return;
+      }
+    }
+    launch_hop_links<D, R, EPI, false>(a, s);
   }
 }
 

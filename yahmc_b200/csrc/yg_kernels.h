@@ -17,6 +17,7 @@ struct HopArgs {
   Geom g;
   const cplx<R> *src;
   const cplx<R> *U;
+  const R *Ur;            // the real links of an adjoint representation (FP64 hop), else null
   cplx<R> *dst;
   cplx<R> *dst2;          // CLOVINV: also store the raw hop here (the reference's in-place write)
   const cplx<R> *src2;    // CLOVADD / AXPY: psi at the output site
@@ -66,7 +67,9 @@ struct DK {
 // Representation map and clover-term build: fundamental N x N links -> D x D
 template <int NC, int D>
 struct RK {
-  static void represent(double2 *links, const double2 *fund, Geom g, const double2 *basis, int rep, cudaStream_t s);
+  // real: also the real parts alone, when not null (adjoint representations)
+  static void represent(double2 *links, double *real, const double2 *fund, Geom g, const double2 *basis, int rep,
+                        cudaStream_t s);
   static void clover_term(double2 *cl, const double2 *fund, Geom g, const double2 *basis, int rep, double csw,
                           cudaStream_t s);
 };

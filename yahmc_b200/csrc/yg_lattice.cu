@@ -51,7 +51,7 @@ Lattice::~Lattice() {
   }
   for (DevBuf *b : {&fund, &links, &clover, &ldl, &cl_force, &mom, &tables, &red_partial, &red_result, &links_f,
                     &clover_f, &cinv_f, &sl_links, &sl_clover, &cpk64, &sl_part, &sl_scal, &fund_backup, &sl_cnorm,
-                    &mr_work, &mr_scal, &mr_part, &mr_clov, &cg_work})
+                    &mr_work, &mr_scal, &mr_part, &mr_clov, &cg_work, &links_r})
     b->release();
 }
 
@@ -235,7 +235,8 @@ __global__ void k_spinor_to_host(double *dst, const double2 *src, Geom g, int d)
 
 // ------------------------------------------------------------------ gauge field
 void represent_and_clover(Lattice &L) {
-  YG_DISPATCH_ND(L.nc, L.d, K::represent(L.links.as<double2>(), L.fund.as<double2>(), L.g, L.rt.basis, L.p.repr, L.stream));
+  YG_DISPATCH_ND(L.nc, L.d, K::represent(L.links.as<double2>(), L.links_r.as<double>(), L.fund.as<double2>(), L.g,
+                                          L.rt.basis, L.p.repr, L.stream));
   YG_LAUNCHED();
   if (L.p.clover) {
     YG_DISPATCH_ND(L.nc, L.d, K::clover_term(L.clover.as<double2>(), L.fund.as<double2>(), L.g, L.rt.basis, L.p.repr,
@@ -303,6 +304,7 @@ Lattice *lattice_create(const yg_params &p) {
     int nc = p.nc, ng = L->ng;
     L->fund.alloc(sizeof(double2) * 4 * V * nc * nc);
     L->links.alloc(sizeof(double2) * 4 * V * d * d);
+    if (p.repr == YG_REPR_ADJOINT) L->links_r.alloc(sizeof(double) * 4 * V * d * d);
     YG_CUDA(cudaMemset(L->fund.p, 0, L->fund.bytes));
     YG_CUDA(cudaMemset(L->links.p, 0, L->links.bytes));
     if (p.clover) {

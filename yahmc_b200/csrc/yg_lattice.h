@@ -61,6 +61,7 @@ struct Lattice {
   DevBuf fund;      // fundamental links, 4 x N x N per site        (gfield_fund)
   DevBuf fund_backup;  // gauge_field_backup copy of fund
   DevBuf links;     // represented links with the AP sign, 4 x d x d (gfield_repr)
+  DevBuf links_r;   // their real parts for the FP64 hop (adjoint representations, whose links are real)
   DevBuf clover;    // clover term, 4 x d x d per site                (cl_term)
   DevBuf ldl;       // LDL factors, 2 x d(2d+1) per site of block 1   (cl_ldl)
   double ldl_sigma = 0;

@@ -101,7 +101,7 @@ __device__ void represent_one(double2 (&r)[D * D], const double2 (&u)[NC * NC], 
 }
 
 template <int NC, int D>
-__global__ void k_represent(double2 *links, const double2 *fund, Geom g, const double2 *basis, int rep) {
+__global__ void k_represent(double2 *links, double *real, const double2 *fund, Geom g, const double2 *basis, int rep) {
   long r = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (r >= 4L * g.V) return;
   int id = (int)(r >> 2), mu = (int)(r & 3);
@@ -112,7 +112,11 @@ __global__ void k_represent(double2 *links, const double2 *fund, Geom g, const d
   int c[4];
   coords_of(g, id, c);
   double sgn = (g.bc == YG_BC_ANTIPERIODIC && mu == 0 && c[0] == 0) ? -1.0 : 1.0;   // bcs.cpp:264-272
-  for (int k = 0; k < D * D; k++) links[fidx(g, id, mu * D * D + k, 4 * D * D)] = cscale(R[k], sgn);
+  for (int k = 0; k < D * D; k++) {
+    const long ix = fidx(g, id, mu * D * D + k, 4 * D * D);
+    links[ix] = cscale(R[k], sgn);
+    if (real) real[ix] = sgn * R[k].x;
+  }
 }
 
 // clover_repr(id,mu,nu) (wilsonloop.cpp:5-31) in the fermion representation: each leaf is a chain
@@ -251,8 +255,9 @@ __global__ void k_clover_term(double2 *cl, const double2 *fund, Geom g, const do
 }
 
 template <int NC, int D>
-void RK<NC, D>::represent(double2 *links, const double2 *fund, Geom g, const double2 *basis, int rep, cudaStream_t s) {
-  k_represent<NC, D><<<nblk(4L * g.V, 128), 128, 0, s>>>(links, fund, g, basis, rep);
+void RK<NC, D>::represent(double2 *links, double *real, const double2 *fund, Geom g, const double2 *basis, int rep,
+                          cudaStream_t s) {
+  k_represent<NC, D><<<nblk(4L * g.V, 128), 128, 0, s>>>(links, real, fund, g, basis, rep);
 }
 
 template <int NC, int D>
