@@ -18,12 +18,12 @@
 // with a barrier of the group after each phase.  Hphi is Hermitian on these lattices (no open or
 // SF slices), so <p, Hphi_sq p> = |Hphi p|^2 and alpha is known before the second Hphi ends, which
 // leaves five barriers an iteration and no pass over q.  The operator steps are the FP64 Schur
-// steps of the single-lattice path (yg_dirac_impl.cuh: four lanes a site up to kQuadSites) with ordinary loads for the
-// fields, which the kernel also writes.  The scalars are the reference's: alpha = rr / <p,q>, beta = rr_new / rr, stop when
-// rr_new < prec |b|^2, iteration count as cg_inverter's.  Reductions are deterministic: one
-// partial per block, which every block of the group adds in block order after the barrier,
-// so all blocks of a group hold the same alpha and beta.  Groups never wait for each other:
-// a lattice that converges early just ends its blocks.
+// steps of the single-lattice path (yg_dirac_impl.cuh: four lanes a site up to kQuadSites) with
+// ordinary loads for the fields, which the kernel also writes.  The scalars are the reference's:
+// alpha = rr / <p,q>, beta = rr_new / rr, stop when rr_new < prec |b|^2, iteration count as
+// cg_inverter's.  Reductions are deterministic: one partial per block, which every block of the
+// group adds in block order after the barrier, so all blocks of a group hold the same alpha and
+// beta.  Groups never wait for each other: a lattice that converges early just ends its blocks.
 //
 // Barriers: one arrival counter per group, on a line of its own, that only grows; a block
 // releases its writes with its arrival and acquires the others' by polling the counter up to the
@@ -46,8 +46,9 @@ namespace yg {
 namespace {
 
 // Two persistent grids at once could each hold multiprocessors that the other one's blocks need: one
-// runs at a time in a process.
-std::mutex g_persistent;
+// runs at a time on a device, as far as this process goes.
+constexpr int kMaxDevices = 64;
+std::mutex g_persistent[kMaxDevices];
 
 constexpr int kThreads = 128;
 constexpr int kSyncStride = 32;                     // words between the groups' counters: 128 bytes
@@ -368,7 +369,7 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
   cudaStream_t s = L[0]->stream;
   int err = 0;
   std::vector<BOut> res(n);
-  std::lock_guard<std::mutex> one(g_persistent);
+  std::lock_guard<std::mutex> one(g_persistent[L[0]->device % kMaxDevices]);
   try {
     YG_CUDA(cudaMemsetAsync(base, 0, bytes, s));
     const long long limit = wait_cycles > 0 ? wait_cycles : kDefaultWait;

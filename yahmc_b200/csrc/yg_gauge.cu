@@ -187,7 +187,9 @@ __device__ __forceinline__ void staple_side(double2 (&st)[N * N], const double2 
 // mom(x,mu) -= algebra_project(U(x,mu) (c0 S_plaq + c1 S_rect), coeff); IMP = 0 skips the
 // rectangles (wilson_gauge_force, c0 = 1).  A block takes 32 sites and one direction, one warp
 // per plane: every link load of a warp is a contiguous run, three threads share a link's chain
-// of products, and their algebra components meet in shared memory.
+// of products, and their algebra components meet in shared memory.  Bound by FP64 latency at 12 warps
+// an SM (168 registers).  SU(3) 32 x 16^3, Symanzik / Wilson: 619 / 181 us; one thread a link, path by
+// path: 1270 / 489.
 template <int N, int IMP>
 __global__ void __launch_bounds__(96, (N <= 3 ? 4 : 2))
     k_gauge_force(double *mom, const double2 *U, Geom g, double coeff, double c0, double c1) {
