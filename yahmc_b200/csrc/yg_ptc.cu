@@ -56,8 +56,17 @@ __host__ __device__ __forceinline__ uint32_t kmajor_off(int r, int k, int K) {
   return (uint32_t)((r >> 3) * (K >> 3) * 128 + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
 }
 
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, int K) {
-  const uint64_t lbo = 128 >> 4, sbo = (uint64_t)((K >> 3) * 128) >> 4;
+// The weight gradient's operands are written two bytes at a time, neighbouring lanes along K: with
+// the K-direction core matrices 128 bytes apart, the four that a warp touches share their banks, so
+// they are put 144 bytes apart there (LBO = 144); with the layers' 16-byte stores of channel pairs the
+// gradients of two pairs on 32 x 16^3 take 4.02 ms, 4.24 before.
+constexpr int kGradCore = 144;
+__host__ __device__ __forceinline__ uint32_t grad_off(int r, int k, int K) {
+  return (uint32_t)((r >> 3) * (K >> 3) * kGradCore + (k >> 3) * kGradCore + (r & 7) * 16 + (k & 7) * 2);
+}
+
+__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, int K, int core = 128) {
+  const uint64_t lbo = core >> 4, sbo = (uint64_t)((K >> 3) * core) >> 4;
   return (uint64_t)((saddr >> 4) & 0x3fff) | (lbo << 16) | (sbo << 32) | (1ull << 46);   // version 1, no swizzle
 }
 
@@ -184,6 +193,19 @@ __device__ __forceinline__ void put_bf16x4(unsigned char *base, uint32_t off, fl
   *reinterpret_cast<uint2 *>(base + off) = w;
 }
 
+// eight consecutive BF16 (one core-matrix row, 16 bytes): k0 a multiple of 8
+__device__ __forceinline__ void put_bf16x8(unsigned char *base, uint32_t off, float v0, float v1, float v2, float v3,
+                                           float v4, float v5, float v6, float v7) {
+  __nv_bfloat162 a = __floats2bfloat162_rn(v0, v1), b = __floats2bfloat162_rn(v2, v3);
+  __nv_bfloat162 c = __floats2bfloat162_rn(v4, v5), d = __floats2bfloat162_rn(v6, v7);
+  uint4 w;
+  w.x = *reinterpret_cast<uint32_t *>(&a);
+  w.y = *reinterpret_cast<uint32_t *>(&b);
+  w.z = *reinterpret_cast<uint32_t *>(&c);
+  w.w = *reinterpret_cast<uint32_t *>(&d);
+  *reinterpret_cast<uint4 *>(base + off) = w;
+}
+
 // Activations are site blocks: channel ch of site id is 24 floats at (ch * V + id) * 24, float
 // k2 = (spin * 3 + colour) * 2 + re/im.  A thread gathers whole blocks with 16-byte loads.
 struct Block {
@@ -297,30 +319,40 @@ __global__ void __launch_bounds__(kThreads, 1) k_ptc_layer(PtcArgs a) {
       const int nid = live ? path_site(a.g, id, c, p) : 0;
       float2 u[9];
       if (live && p > 0) path_link(a, id, nid, p, u);
-      constexpr int NCH = CI >= NPART ? CI / NPART : 1;     // channels per thread
+      constexpr int NCH = CI >= NPART ? CI / NPART : 1;     // channels per thread, part * NCH ...
       constexpr int CB = NCH < 4 ? NCH : 4;                  // gathered together
+      constexpr int PW = CB < 2 ? 1 : 2;                     // stored together: eight columns, 16 bytes
 #pragma unroll 1
       for (int c0 = 0; c0 < NCH; c0 += CB) {
+        const int ch0 = CI >= NPART ? part * NCH + c0 : 0;
         Block f[CB];
 #pragma unroll
         for (int q = 0; q < CB; q++) {
-          const int ch = CI >= NPART ? part + NPART * (c0 + q) : 0;
-          if (live) load_block(f[q], a.in, (long)ch * a.V + nid);
+          if (live) load_block(f[q], a.in, (long)(ch0 + q) * a.V + nid);
           else
 #pragma unroll
             for (int k = 0; k < 6; k++) f[q].w[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
-        for (int q = 0; q < CB; q++) {
-          const int ch = CI >= NPART ? part + NPART * (c0 + q) : 0;
-          float2 y[4][3];
-          if (p == 0) transport_block<true>(y, f[q], u);
-          else transport_block<false>(y, f[q], u);
+        for (int q = 0; q < CB; q += PW) {
+          float2 y[PW][4][3];
+#pragma unroll
+          for (int e = 0; e < PW; e++) {
+            if (p == 0) transport_block<true>(y[e], f[q + e], u);
+            else transport_block<false>(y[e], f[q + e], u);
+          }
 #pragma unroll
           for (int cl = 0; cl < 3; cl++) {
-            const int r = cl * kTileSites + j;
-            put_bf16x4(B, kmajor_off(r, ch * 4, KP), y[0][cl].x, y[1][cl].x, y[2][cl].x, y[3][cl].x);
-            put_bf16x4(B, kmajor_off(r, PAIRS + ch * 4, KP), y[0][cl].y, y[1][cl].y, y[2][cl].y, y[3][cl].y);
+            const int r = cl * kTileSites + j, k0 = (ch0 + q) * 4;
+            if constexpr (PW == 2) {
+              put_bf16x8(B, kmajor_off(r, k0, KP), y[0][0][cl].x, y[0][1][cl].x, y[0][2][cl].x, y[0][3][cl].x,
+                         y[1][0][cl].x, y[1][1][cl].x, y[1][2][cl].x, y[1][3][cl].x);
+              put_bf16x8(B, kmajor_off(r, PAIRS + k0, KP), y[0][0][cl].y, y[0][1][cl].y, y[0][2][cl].y, y[0][3][cl].y,
+                         y[1][0][cl].y, y[1][1][cl].y, y[1][2][cl].y, y[1][3][cl].y);
+            } else {
+              put_bf16x4(B, kmajor_off(r, k0, KP), y[0][0][cl].x, y[0][1][cl].x, y[0][2][cl].x, y[0][3][cl].x);
+              put_bf16x4(B, kmajor_off(r, PAIRS + k0, KP), y[0][0][cl].y, y[0][1][cl].y, y[0][2][cl].y, y[0][3][cl].y);
+            }
           }
         }
       }
@@ -392,7 +424,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_ptc_layer(PtcArgs a) {
 // of [C_re | C_im], padded to NB; same K) in shared memory: PG paths share the 128 rows of one product
 // (9, 3 or 2 paths for 1, 8 or 16 input channels), each gathered by its own threads, where one path at
 // a time left 3/4 of the rows empty and 128 threads a SM (8-1, 8-8, 1-8 on 32 x 16^3: 505, 723, 533 us;
-// now 177, 408, 93).  The CTA accumulates its tiles in tensor
+// then 177, 408, 93).  The CTA accumulates its tiles in tensor
 // memory and writes one partial per path.
 template <int CI> struct WgradCfg {
   static constexpr int PG = CI == 1 ? 9 : CI == 8 ? 3 : 2;      // paths per product
@@ -409,9 +441,10 @@ __global__ void __launch_bounds__(WgradCfg<CI>::threads, 1) k_ptc_wgrad(PtcArgs 
   constexpr int NB = ((2 * CO * 4 + 15) / 16) * 16;       // GEMM columns
   constexpr int PAIRS = CI * 4, OPAIRS = CO * 4;
   extern __shared__ __align__(1024) unsigned char sm[];
+  constexpr int ABYTES = kM / 8 * (KW / 8) * kGradCore, BBYTES = NB / 8 * (KW / 8) * kGradCore;
   unsigned char *sA = sm;                                 // kM x KW (transported inputs)
-  unsigned char *sB = sm + kM * KW * 2;                   // NB x KW (output gradients)
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(sB + NB * KW * 2);
+  unsigned char *sB = sm + ABYTES;                        // NB x KW (output gradients)
+  uint64_t *mbar = reinterpret_cast<uint64_t *>(sB + BBYTES);
   uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + 1);
   constexpr int cols = NB <= 32 ? 32 : NB <= 64 ? 64 : 128;
   static_assert(PG * PAIRS <= kM && NB <= 128, "one product per tile");
@@ -422,9 +455,9 @@ __global__ void __launch_bounds__(WgradCfg<CI>::threads, 1) k_ptc_wgrad(PtcArgs 
   if (tid == 0) mbar_init(smem_u32(mbar));
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   // rows of A beyond the paths' input pairs stay zero (the last group of two paths has one)
-  for (int e = tid; e < kM * KW * 2 / 16; e += NT) reinterpret_cast<uint4 *>(sA)[e] = make_uint4(0, 0, 0, 0);
+  for (int e = tid; e < ABYTES / 16; e += NT) reinterpret_cast<uint4 *>(sA)[e] = make_uint4(0, 0, 0, 0);
   for (int e = tid; e < (NB - 2 * OPAIRS) * KW; e += NT)
-    put_bf16(sB, kmajor_off(2 * OPAIRS + e / KW, e % KW, KW), 0.f);
+    put_bf16(sB, grad_off(2 * OPAIRS + e / KW, e % KW, KW), 0.f);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -450,10 +483,10 @@ __global__ void __launch_bounds__(WgradCfg<CI>::threads, 1) k_ptc_wgrad(PtcArgs 
         for (int c = 0; c < 3; c++) {
           const float2 gv = blk_c(gb, sp, c);
           const int os = o * 4 + sp, n = c * kTileSites + jj;
-          put_bf16(sB, kmajor_off(os, n, KW), gv.x);
-          put_bf16(sB, kmajor_off(os, kN + n, KW), gv.y);
-          put_bf16(sB, kmajor_off(OPAIRS + os, n, KW), -gv.y);
-          put_bf16(sB, kmajor_off(OPAIRS + os, kN + n, KW), gv.x);
+          put_bf16(sB, grad_off(os, n, KW), gv.x);
+          put_bf16(sB, grad_off(os, kN + n, KW), gv.y);
+          put_bf16(sB, grad_off(OPAIRS + os, n, KW), -gv.y);
+          put_bf16(sB, grad_off(OPAIRS + os, kN + n, KW), gv.x);
         }
     }
     if (p < kPaths) {
@@ -488,8 +521,8 @@ __global__ void __launch_bounds__(WgradCfg<CI>::threads, 1) k_ptc_wgrad(PtcArgs 
 #pragma unroll
             for (int cl = 0; cl < 3; cl++) {
               const int n = cl * kTileSites + j, row = pp * PAIRS + ch * 4 + sp;
-              put_bf16(sA, kmajor_off(row, n, KW), y[sp][cl].x);
-              put_bf16(sA, kmajor_off(row, kN + n, KW), y[sp][cl].y);
+              put_bf16(sA, grad_off(row, n, KW), y[sp][cl].x);
+              put_bf16(sA, grad_off(row, kN + n, KW), y[sp][cl].y);
             }
         }
       }
@@ -502,7 +535,8 @@ __global__ void __launch_bounds__(WgradCfg<CI>::threads, 1) k_ptc_wgrad(PtcArgs 
       const uint32_t aa = smem_u32(sA), bb = smem_u32(sB);
 #pragma unroll 4
       for (int kk = 0; kk < KW / 16; kk++)
-        mma_bf16(tmem, smem_desc(aa + kk * 256, KW), smem_desc(bb + kk * 256, KW), idesc_bf16(kM, NB),
+        mma_bf16(tmem, smem_desc(aa + kk * 2 * kGradCore, KW, kGradCore),
+                 smem_desc(bb + kk * 2 * kGradCore, KW, kGradCore), idesc_bf16(kM, NB),
                  (tile != (int)blockIdx.x || kk > 0) ? 1u : 0u);
       mma_commit(smem_u32(mbar));
     }
@@ -666,7 +700,9 @@ size_t layer_smem() {
   return std::max(kMinSmem, (size_t)LayerBufs<CI>::value * ((size_t)(kM + kN) * kp_of(CI) * 2 + 16) + 16);
 }
 template <int CI, int CO>
-size_t wgrad_smem() { return (size_t)kM * 2 * kN * 2 + (size_t)(((2 * CO * 4 + 15) / 16) * 16) * 2 * kN * 2 + 16; }
+size_t wgrad_smem() {
+  return (size_t)(kM + ((2 * CO * 4 + 15) / 16) * 16) / 8 * (2 * kN / 8) * kGradCore + 16;
+}
 
 template <int CI, int CO>
 void run_layer(Lattice &L, const PtcArgs &a) {
