@@ -353,6 +353,9 @@ int yg_ptc_set_weights(yg_ptc *net, int layer, const double *w);
 int yg_ptc_get_weights(yg_ptc *net, int layer, double *w);
 /* one layer on device activations; adjoint = 1: the input-gradient layer (Co -> Ci) */
 int yg_ptc_layer(yg_ptc *net, int layer, int adjoint, const float *dev_in, float *dev_out);
+/* polls after which a wait inside the network's kernels gives up (negative: the default).  A kernel
+ * whose wait ran out ends its own copies and products and the call returns YG_TIMEOUT. */
+int yg_ptc_wait_limit(yg_ptc *net, long polls);
 /* dst (even sites) = the network applied to the even-site field src embedded with zero odd
  * sites (the even-even block of D^-1 is the inverse of the Schur operator Dphi) */
 int yg_ptc_apply(yg_ptc *net, double *dst, const double *src);

@@ -162,3 +162,31 @@ def test_trained_network_cuts_fgcr_iterations():
     for st in (plain, start, trained):
         assert st["status"] == 0 and st["fallback"] == 0 and st["true_residual"] < prec
     assert trained["iterations"] < plain["iterations"], (trained, start, plain)
+
+
+@pytest.mark.parametrize("channels", [(1, 8, 8, 1), (1, 16, 16, 1)])
+def test_wait_that_runs_out_is_reported_and_leaves_the_network_usable(channels):
+    """With a limit of no polls every wait in the kernels runs out: they end their own copies and
+    products, each call reports the status, and later calls give the results of before."""
+    import torch
+    from yahmc_b200 import Ptc, YGError
+    lat, O, rng = make_pair("su3_fund_ap", (4, 6, 6, 6), seed=31)
+    net = Ptc(lat, channels)
+    net.set_weights([0.05 * _rand(rng, s) for s in net.shapes()])
+    src, dst = lat.field(source(O, rng)), lat.field()
+    act = torch.zeros(24 * O.V * max(channels), device="cuda")
+    out = torch.zeros_like(act)
+    calls = [lambda: net.apply(dst, src), lambda: net.gradient([(src, src)]), lambda: net.backward(src, src),
+             lambda: net.layer(1, 0, act.data_ptr(), out.data_ptr())]
+    net.apply(dst, src)
+    before, grads = lat.download(dst), net.gradient([(src, src)])
+    net.wait_limit(0)
+    for call in calls:
+        with pytest.raises(YGError) as e:
+            call()
+        assert e.value.code == 7
+    net.wait_limit()
+    net.apply(dst, src)
+    assert np.array_equal(lat.download(dst)[:O.Vh], before[:O.Vh])
+    loss, again = net.gradient([(src, src)])
+    assert loss == grads[0] and all(np.array_equal(a, b) for a, b in zip(again, grads[1]))

@@ -130,7 +130,7 @@ _SIGNATURES = {
     "yg_field_sqnorm_noalloc": [_P, ctypes.c_long, _P, _P],
     "yg_wilson_fermion_force_q_multi": [_P, _D, _D, _I, _P, _P],
     "yg_ptc_create": [_P, _I, _P, _P], "yg_ptc_destroy": [_P], "yg_ptc_set_weights": [_P, _I, _P],
-    "yg_ptc_get_weights": [_P, _I, _P], "yg_ptc_layer": [_P, _I, _I, _P, _P], "yg_ptc_apply": [_P, _P, _P],
+    "yg_ptc_get_weights": [_P, _I, _P], "yg_ptc_layer": [_P, _I, _I, _P, _P], "yg_ptc_wait_limit": [_P, ctypes.c_long], "yg_ptc_apply": [_P, _P, _P],
     "yg_ptc_gradient": [_P, _I, _P, _P, _P, _P], "yg_ptc_backward": [_P, _P, _P, _P],
     "yg_fgcr": [_P, _P, ctypes.POINTER(InvPar), _I, _P, _P, ctypes.POINTER(SolveStats)],
     "yg_solve_learned": [_P, _P, ctypes.POINTER(InvPar), _I, _P, _P, ctypes.POINTER(SolveStats)],
@@ -213,6 +213,10 @@ class Ptc:
         """One layer on device activations (site blocks; raw device pointers)."""
         self.lat._check(self.lib.yg_ptc_layer(self.h, int(l), int(adjoint), ctypes.c_void_p(dev_in),
                                               ctypes.c_void_p(dev_out)))
+
+    def wait_limit(self, polls=-1):
+        """Polls after which a wait inside the kernels gives up and the call reports YG_TIMEOUT."""
+        self.lat._check(self.lib.yg_ptc_wait_limit(self.h, int(polls)))
 
     def apply(self, dst, src):
         self.lat._check(self.lib.yg_ptc_apply(self.h, dst.ptr, src.ptr))

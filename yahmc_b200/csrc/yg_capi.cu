@@ -460,10 +460,11 @@ int yg_ptc_layer(yg_ptc *h, int layer, int adjoint, const float *in, float *out)
   return guard([&] {
     need(in, "in");
     need(out, "out");
-    yg::Ptc &n = ptc(h);
-    yg::ptc_layer(n, layer, adjoint, in, out);
-    YG_CUDA(cudaStreamSynchronize(yg::ptc_lattice(n).stream));
+    yg::ptc_layer(ptc(h), layer, adjoint, in, out);
   });
+}
+int yg_ptc_wait_limit(yg_ptc *h, long polls) {
+  return guard([&] { yg::ptc_wait_limit(ptc(h), polls); });
 }
 int yg_ptc_apply(yg_ptc *h, double *dst, const double *src) {
   return guard([&] { need(dst, "dst"); need(src, "src"); yg::ptc_apply(ptc(h), dst, src); });

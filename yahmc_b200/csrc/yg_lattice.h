@@ -295,10 +295,10 @@ constexpr int kPtcMaxLayers = 8;
 struct Ptc;
 Ptc *ptc_create(Lattice &L, int nl, const int *ch);
 void ptc_destroy(Ptc *n);
-Lattice &ptc_lattice(Ptc &n);
 void ptc_set_weights(Ptc &n, int l, const double *w);
 void ptc_get_weights(Ptc &n, int l, double *w);
 void ptc_layer(Ptc &n, int l, int adjoint, const float *in, float *out);
+void ptc_wait_limit(Ptc &n, long polls);
 void ptc_apply(Ptc &n, double *dst, const double *src);
 double ptc_gradient(Ptc &n, int npairs, double *const *r, double *const *e, double *grads);
 void ptc_backward(Ptc &n, const double *src, const double *gout, double *grads);

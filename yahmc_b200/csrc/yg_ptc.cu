@@ -96,8 +96,8 @@ __device__ __forceinline__ void mbar_init(uint32_t mbar) {
 }
 
 // waits for phase `phase` of the barrier; false if the bounded wait ran out
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase) {
-  for (long i = 0; i < kSpinLimit; i++) {
+__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase, long limit = kSpinLimit) {
+  for (long i = 0; i < limit; i++) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
@@ -154,6 +154,7 @@ struct PtcArgs {
   const float *gin;         // wgrad: Co channels of output gradient planes
   float *part;              // wgrad: per-CTA partial weight gradients
   int *err;                 // bounded-wait failures
+  long polls;               // limit of each wait (kSpinLimit; a test's 0 makes every wait run out)
   int V;
   int nout;                 // sites of the output that are wanted: [0, nout), V or the even half
   int in_even;              // the input vanishes on odd sites: a site's own path or its eight hops carry nothing
@@ -292,6 +293,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_ptc_layer(PtcArgs a) {
   tc_fence_after();
   const uint32_t tmem = *tslot;
   bool ok = true, good = true;      // the block's, and this thread's waits
+  int copies = 0, products = 0;     // thread 0: bulk copies and products issued
 
   constexpr int NPART = kThreads / kTileSites;
   const int j = tid % kTileSites, part = tid / kTileSites;
@@ -311,8 +313,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_ptc_layer(PtcArgs a) {
     const uint32_t mma_bar = smem_u32(mbar + buf), w_bar = smem_u32(mbar + NBUF + buf);
     unsigned char *B = sB + buf * BBYTES;
     // the buffers' last product is done; a wait that runs out ends the loop for all at the next barrier
-    if (i >= NBUF) good = mbar_wait(mma_bar, (uint32_t)((i / NBUF - 1) & 1)) && good;
-    if (tid == 0 && good) bulk_load(smem_u32(sA + buf * ABYTES), a.A + (long)p * kM * KP, AUSED, w_bar);
+    if (i >= NBUF) good = mbar_wait(mma_bar, (uint32_t)((i / NBUF - 1) & 1), a.polls) && good;
+    if (tid == 0 && good) {
+      bulk_load(smem_u32(sA + buf * ABYTES), a.A + (long)p * kM * KP, AUSED, w_bar);
+      copies = i + 1;
+    }
     // B chunk: the transported inputs of the tile's sites.  Thread (site j, part) takes the
     // channels part, part + NPART, ...; a one-channel input is gathered by part 0.
     if (CI >= NPART || part == 0) {
@@ -361,7 +366,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_ptc_layer(PtcArgs a) {
     tc_fence_before();
     ok = __syncthreads_and(good);
     if (tid == 0 && ok) {
-      good = mbar_wait(w_bar, (uint32_t)((i / NBUF) & 1));
+      good = mbar_wait(w_bar, (uint32_t)((i / NBUF) & 1), a.polls);
       tc_fence_after();
       if (good) {
         const uint32_t aa = smem_u32(sA + buf * ABYTES), bb = smem_u32(B);
@@ -370,14 +375,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_ptc_layer(PtcArgs a) {
           mma_bf16(tmem, smem_desc(aa + kk * 256, KP), smem_desc(bb + kk * 256, KP), idesc_bf16(kM, kN),
                    (i > 0 || kk > 0) ? 1u : 0u);
         mma_commit(mma_bar);
+        products = i + 1;
       }
     }
   }
   // the last product of each buffer: products complete in order, so the last one implies the others
-  if (ok && good) good = mbar_wait(smem_u32(mbar + (np - 1) % NBUF), (uint32_t)(((np - 1) / NBUF) & 1));
+  if (ok && good) good = mbar_wait(smem_u32(mbar + (np - 1) % NBUF), (uint32_t)(((np - 1) / NBUF) & 1), a.polls);
   if (!good) atomicExch(a.err, 1);
-  tc_fence_after();
   ok = __syncthreads_and(ok && good);
+  // after a wait that ran out: shared and tensor memory are given back only once the copies and products
+  // still in flight have ended
+  if (!ok && tid == 0) {
+    if (copies) mbar_wait(smem_u32(mbar + NBUF + (copies - 1) % NBUF), (uint32_t)(((copies - 1) / NBUF) & 1));
+    if (products) mbar_wait(smem_u32(mbar + (products - 1) % NBUF), (uint32_t)(((products - 1) / NBUF) & 1));
+  }
+  tc_fence_after();
 
   if (ok) {
     // epilogue: accumulator row m = (o, s) real part (m < 4 CO) or imaginary part
@@ -540,11 +552,12 @@ __global__ void __launch_bounds__(WgradCfg<CI>::threads, 1) k_ptc_wgrad(PtcArgs 
                  (tile != (int)blockIdx.x || kk > 0) ? 1u : 0u);
       mma_commit(smem_u32(mbar));
     }
-    ok = mbar_wait(smem_u32(mbar), phase);
-    phase ^= 1u;
-    if (!ok && tid == 0) atomicExch(a.err, 1);
-    tc_fence_after();
+    ok = mbar_wait(smem_u32(mbar), phase, a.polls);
+    if (!ok) atomicExch(a.err, 1);
     ok = __syncthreads_and(ok);
+    if (!ok && tid == 0) mbar_wait(smem_u32(mbar), phase);      // the product still in flight
+    phase ^= 1u;
+    tc_fence_after();
   }
 
   if (ok && warp < 4) {
@@ -642,6 +655,7 @@ struct Ptc {
   DevBuf g[2];                          // gradient ping-pong
   DevBuf part, err, dpart, wsum;
   int maxc = 1;
+  long polls = kSpinLimit;              // limit of the kernels' waits
 };
 
 namespace {
@@ -742,6 +756,7 @@ PtcArgs base_args(Ptc &n) {
   a.U = n.L->links.as<double2>();
   a.err = n.err.as<int>();
   a.V = a.nout = (int)n.L->V;
+  a.polls = n.polls;
   return a;
 }
 
@@ -788,7 +803,6 @@ Ptc *ptc_create(Lattice &L, int nl, const int *ch) {
   return n;
 }
 
-Lattice &ptc_lattice(Ptc &n) { return *n.L; }
 
 void ptc_destroy(Ptc *n) {
   if (!n) return;
@@ -837,7 +851,10 @@ static void layer(Ptc &n, int l, int adjoint, const float *in, float *out, bool 
 void ptc_layer(Ptc &n, int l, int adjoint, const float *in, float *out) {
   if (l < 0 || l >= n.nl) throw Error(YG_ERR_ARG, "layer index");
   layer(n, l, adjoint, in, out, false, false);
+  check_err(n);
 }
+
+void ptc_wait_limit(Ptc &n, long polls) { n.polls = polls < 0 ? kSpinLimit : polls; }
 
 // forward through all layers from act[0]; act[l] keeps every layer's input, act[nl] the output on the
 // even sites
