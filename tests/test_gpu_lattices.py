@@ -124,3 +124,38 @@ def test_errors():
     b = lat.field(source(O, rng))
     with pytest.raises(YGError):
         cg_inverter_lattices([(lat, -0.4, 1e-20, lat.field(), b), (lat, -0.4, 1e-20, lat.field(), b)])
+
+
+def test_persistent_solve_goes_on_over_several_launches():
+    """One launch makes at most 1000 iterations: an ill-conditioned system (smallest eigenvalues of
+    Hphi_sq near 1e-6 on random links) needs more, so the solve goes on in further launches, and ends where
+    its true residual meets prec, or at exactly maxiter."""
+    from yahmc_b200 import cg_inverter_lattices, launch_count
+    lat, O, rng = make_pair("su3_fund_ap", (4, 4, 4, 4), seed=23)
+    b0 = source(O, rng)
+    b, x = lat.field(b0), lat.field()
+    lat.cg_inverter("Hphi_sq", -2.3, 1e-14, x, b, maxiter=10)
+    lat.spinor_zero(x)
+    n0 = launch_count()
+    assert lat.cg_inverter("Hphi_sq", -2.3, 1e-14, x, b, maxiter=10) == 10
+    n10 = launch_count() - n0
+    lat.spinor_zero(x)
+    n0 = launch_count()
+    it = lat.cg_inverter("Hphi_sq", -2.3, 1e-14, x, b)
+    assert it > 2000
+    assert launch_count() - n0 == n10 + (it - 1) // 1000
+    q, xs = O.new_field(), lat.download(x)
+    O.Hphi_sq(-2.3, q, xs)
+    r = (q - b0)[:O.Vh]
+    # the recursive residual meets prec; the true one differs by the rounding of A x: 1.1e-16 times the
+    # largest eigenvalue (below 100) times |x| (2e5 |b| here), 2e-9 |b|, so by 2 * 1e-7 * 2e-9 |b|^2 at most
+    assert np.vdot(r, r).real < 1.1e-14 * np.vdot(b0[:O.Vh], b0[:O.Vh]).real
+    # a batch in which one lattice ends in the first launch and one stops at maxiter in the third
+    lat2, O2, rng2 = make_pair("su3_fund_ap", (4, 4, 4, 6), seed=24)
+    b2, x2, x2s = lat2.field(source(O2, rng2)), lat2.field(), lat2.field()
+    it2 = lat2.cg_inverter("Hphi_sq", 0.2, 1e-22, x2s, b2)
+    lat.spinor_zero(x)
+    its, rc, path = cg_inverter_lattices([(lat, -2.3, 0.0, x, b, 2345), (lat2, 0.2, 1e-22, x2, b2)], with_path=True)
+    assert path == 1 and rc == 4 and its[0] == 2345 and abs(its[1] - it2) <= 1
+    got, ref = _even(lat2, x2), _even(lat2, x2s)
+    assert np.abs(got - ref).max() <= 1e-10 * np.abs(ref).max()

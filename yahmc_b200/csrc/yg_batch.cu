@@ -31,7 +31,9 @@
 // wait runs out sets the launch's error flag and returns, every other block meets the flag in its
 // next wait (the missing arrival keeps it there) and returns too, and the host reports YG_TIMEOUT.
 // The launch is cooperative, so all blocks are resident and in a healthy run every barrier
-// completes; the limit is the guard against anything else.
+// completes; the limit is the guard against anything else.  The iterations of one launch are bounded
+// too (launch_iters): a solve that needs more, or never converges, goes on in further launches from the
+// fields and scalars the last one left, so the device and the host get their turn.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -56,6 +58,13 @@ constexpr int kSyncStride = 32;                     // words between the groups'
 constexpr long long kDefaultWait = 20000000000LL;   // cycles (about 10 s at 2 GHz)
 
 constexpr int kMaxLattices = 64;
+
+constexpr int kMore = -1;                           // status of a lattice that goes on in the next launch
+
+// iterations of one launch: at most about 0.1 s of them (3 ns a site and iteration at d = 3, 25 us the
+// least), against some 20 us for another launch
+int launch_iters(long sites) { return (int)std::max(16L, std::min(1000L, 40000000L / sites)); }
+
 constexpr int kSiteMaxD = 4;                        // d = 6 with a thread a site spills under 168 registers
 
 struct BLat {
@@ -64,8 +73,8 @@ struct BLat {
   double2 *x, *r, *p, *t, *o;          // whole-field layout; x, r, p, t even sites, o odd
   int b0, nb;                          // the group's blocks [b0, b0 + nb)
   int quad;                            // four lanes a site instead of one thread
-  int maxiter, it0;                    // it0 = -1: solved by the initial guess, no iteration
-  double diag, target, rr0;            // diagonal of A_ee, prec |b|^2, |r|^2 of the initial residual
+  int maxiter, it0, it1;               // iterations it0 + 1 .. it1 of this launch; it0 = -1: none, the solve has ended
+  double diag, target, rr0;            // diagonal of A_ee, prec |b|^2, |r|^2 after it0 iterations
 };
 
 // A kernel parameter: geometry and pointers stay in the constant bank.  Read from global memory they
@@ -152,9 +161,9 @@ __device__ __forceinline__ void group_cg(const BLat &L, double *part_pq, double 
   e.zero_add_at_boundary = 1;
   unsigned due = 0;
   double rr = L.rr0, alpha = 0.0;
-  int it = 0, status = YG_OK;
+  int it = L.it0, status = YG_OK;
   // cg.cpp:151-153: a system solved by its initial guess returns 0 iterations
-  while (L.it0 == 0 && status == YG_OK) {
+  while (L.it0 >= 0 && status == YG_OK) {
     ++it;
     if (L.maxiter > 0 && it > L.maxiter) { it--; status = YG_MAXITER; break; }
 #pragma unroll 1
@@ -229,7 +238,8 @@ __device__ __forceinline__ void group_cg(const BLat &L, double *part_pq, double 
       }
     }
     if (status != YG_OK || rr < L.target) break;
-    if (!group_sync(cnt, due, nb, err, limit)) status = YG_TIMEOUT;
+    if (it >= L.it1) status = kMore;
+    else if (!group_sync(cnt, due, nb, err, limit)) status = YG_TIMEOUT;
   }
   if (lb == 0 && threadIdx.x == 0) {
     out->iters = it;
@@ -322,6 +332,7 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
   YG_BATCH_D(d, clov, grid_max = resident_blocks<BD, BC>());
   if (grid_max < n) throw Error(YG_ERR_ARG, "more lattices than resident blocks");
   int b0 = 0;
+  std::vector<BOut> fin(n);
   for (int i = 0; i < n; i++) {
     Lattice &l = *L[i];
     const double mass = par[i].mass;
@@ -347,6 +358,7 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
     b.target = norm * par[i].prec;
     b.rr0 = rr;
     b.it0 = rr < b.target ? -1 : 0;
+    fin[i] = BOut{0, YG_OK, rr};
     // blocks in proportion to the even volume, at least one, and no more than the passes over the
     // sites need (fewer blocks make a cheaper barrier)
     const long share = std::max(1L, (long)((double)grid_max * (double)l.Vh / (double)vol));
@@ -367,32 +379,44 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
   L[0]->cg_work.alloc(bytes);            // kept: an allocation would synchronise the device on every solve
   char *base = L[0]->cg_work.as<char>();
   cudaStream_t s = L[0]->stream;
-  int err = 0;
+  int err = 0, step = launch_iters(vol);
+  bool more = true;
   std::vector<BOut> res(n);
   std::lock_guard<std::mutex> one(g_persistent[L[0]->device % kMaxDevices]);
   try {
-    YG_CUDA(cudaMemsetAsync(base, 0, bytes, s));
     const long long limit = wait_cycles > 0 ? wait_cycles : kDefaultWait;
     double *part = reinterpret_cast<double *>(base);
-    YG_BATCH_D(d, clov, launch_batch<BD, BC>(grid, s, args, part, part + grid,
-                                             reinterpret_cast<unsigned *>(base + off_sync),
-                                             reinterpret_cast<int *>(base + off_err),
-                                             reinterpret_cast<BOut *>(base + off_out), limit));
-    YG_CUDA(cudaMemcpyAsync(res.data(), base + off_out, sizeof(BOut) * n, cudaMemcpyDeviceToHost, s));
-    YG_CUDA(cudaMemcpyAsync(&err, base + off_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    YG_CUDA(cudaStreamSynchronize(s));
+    while (more && !err) {
+      for (int i = 0; i < n; i++) h[i].it1 = h[i].it0 + step;
+      YG_CUDA(cudaMemsetAsync(base, 0, bytes, s));
+      YG_BATCH_D(d, clov, launch_batch<BD, BC>(grid, s, args, part, part + grid,
+                                               reinterpret_cast<unsigned *>(base + off_sync),
+                                               reinterpret_cast<int *>(base + off_err),
+                                               reinterpret_cast<BOut *>(base + off_out), limit));
+      YG_CUDA(cudaMemcpyAsync(res.data(), base + off_out, sizeof(BOut) * n, cudaMemcpyDeviceToHost, s));
+      YG_CUDA(cudaMemcpyAsync(&err, base + off_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+      YG_CUDA(cudaStreamSynchronize(s));
+      more = false;
+      for (int i = 0; i < n; i++) {
+        if (h[i].it0 < 0) continue;
+        fin[i] = res[i];
+        h[i].rr0 = res[i].rr;
+        h[i].it0 = res[i].status == kMore ? res[i].iters : -1;
+        more = more || h[i].it0 >= 0;
+      }
+    }
   } catch (...) {
     cudaStreamSynchronize(s);
     throw;
   }
   int worst = YG_OK;
   for (int i = 0; i < n; i++) {
-    iters[i] = res[i].iters;
-    L[i]->mvm += 4 * res[i].iters;
+    iters[i] = fin[i].iters;
+    L[i]->mvm += 4 * fin[i].iters;
     if (par[i].log)
-      fprintf(stderr, "[INVERTER][30]cg: iterations = %d, precision = %1.4e\n", res[i].iters,
-              res[i].rr / (h[i].target / par[i].prec));
-    if (res[i].status != YG_OK && worst == YG_OK) worst = res[i].status;
+      fprintf(stderr, "[INVERTER][30]cg: iterations = %d, precision = %1.4e\n", fin[i].iters,
+              fin[i].rr / (h[i].target / par[i].prec));
+    if (fin[i].status > YG_OK && worst == YG_OK) worst = fin[i].status;
   }
   if (err) return YG_TIMEOUT;
   return worst;
