@@ -159,3 +159,26 @@ def test_persistent_solve_goes_on_over_several_launches():
     assert path == 1 and rc == 4 and its[0] == 2345 and abs(its[1] - it2) <= 1
     got, ref = _even(lat2, x2), _even(lat2, x2s)
     assert np.abs(got - ref).max() <= 1e-10 * np.abs(ref).max()
+
+
+def test_persistent_batch_of_one_large_and_many_tiny_lattices():
+    """63 lattices of 8 even sites beside one of 384 tiles: a block for each tiny lattice and the
+    large one's share stay within the resident grid."""
+    from yahmc_b200 import Lattice, cg_inverter_lattices
+    big = Lattice((24, 16, 16, 16))
+    big.momenta_gaussian(5)
+    big.update_links(0.3)
+    big.represent_gauge_field()
+    bb = big.field(np.random.default_rng(6).standard_normal((big.V, 4, big.d)) + 0j)
+    tiny = [make_pair("su3_fund_ap", (2, 2, 2, 2), seed=200 + k) for k in range(63)]
+    tb = [lat.field(source(O, rng)) for lat, O, rng in tiny]
+    solves = [(big, 0.5, 1e-20, big.field(), bb)]
+    solves += [(lat, 0.5, 1e-20, lat.field(), b) for (lat, _, _), b in zip(tiny, tb)]
+    its, rc, path = cg_inverter_lattices(solves, with_path=True)
+    assert rc == 0 and path == 1
+    for k, (lat, m, prec, x, b) in enumerate(solves):
+        ref = lat.field()
+        itr = lat.cg_inverter_multi("Hphi_sq", m, prec, [ref], [b])[0]
+        assert abs(its[k] - itr) <= 1
+        got, want = _even(lat, x), _even(lat, ref)
+        assert np.abs(got - want).max() <= 1e-9 * np.abs(want).max()

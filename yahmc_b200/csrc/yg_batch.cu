@@ -359,9 +359,9 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
     b.rr0 = rr;
     b.it0 = rr < b.target ? -1 : 0;
     fin[i] = BOut{0, YG_OK, rr};
-    // blocks in proportion to the even volume, at least one, and no more than the passes over the
-    // sites need (fewer blocks make a cheaper barrier)
-    const long share = std::max(1L, (long)((double)grid_max * (double)l.Vh / (double)vol));
+    // one block each, the others in proportion to the even volume (so that all shares together fit the
+    // resident grid), and no more than the passes over the sites need (fewer blocks make a cheaper barrier)
+    const long share = 1 + (grid_max - n) * (long)l.Vh / vol;
     b.quad = d > kSiteMaxD || l.Vh <= kQuadSites;
     const long tiles = nblk(l.Vh, b.quad ? kThreads / 4 : kThreads), passes = (tiles + share - 1) / share;
     b.nb = (int)((tiles + passes - 1) / passes);
