@@ -36,6 +36,7 @@
 // fields and scalars the last one left, so the device and the host get their turn.
 #include <algorithm>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <mutex>
 #include <vector>
@@ -47,12 +48,48 @@ namespace yg {
 
 namespace {
 
-// Two persistent grids at once could each hold multiprocessors that the other one's blocks need: one
-// runs at a time on a device, as far as this process goes.
-constexpr int kMaxDevices = 64;
-std::mutex g_persistent[kMaxDevices];
-
 constexpr int kThreads = 128;
+constexpr int kPerSM = 3;                           // blocks an SM has room for, whatever the instantiation
+
+// Persistent grids that run at once must all fit the device together, or each could hold
+// multiprocessors that another one's blocks need.  So, as far as this process goes, a launch takes a slot
+// for each of its blocks, kPerSM for each SM of the device, and waits, in order of arrival, until enough
+// are free: an SM with fewer than kPerSM blocks has room for one more of any instantiation, so while the
+// blocks of all launches are no more than the slots, each finds a place.  A launch of more blocks than
+// slots (small d) runs alone.  Solves of host threads on lattices of their own, one call each, us for all
+// of them, one launch at a time / sharing the device (cg_launches before this kernel took them):
+//   d = 3, 60 iterations: 8^4 x 4 4962 / 1767 (5533), x 16 19336 / 6370 (11152);
+//   12^4 x 2 5691 / 3196 (6538), x 8 22459 / 11295 (11910), x 16 44696 / 21953 (20651);
+//   16^4 fills the device: x 4 18872 / 18881 (16470), where one alone takes 4935 (8083).
+constexpr int kMaxDevices = 64;
+struct Slots {
+  std::mutex m;
+  std::condition_variable cv;
+  long used = 0;
+  unsigned long next = 0, serving = 0;
+} g_slots[kMaxDevices];
+
+class SlotHold {
+ public:
+  SlotHold(int device, long blocks, long cap) : s(g_slots[device % kMaxDevices]), held(std::min(blocks, cap)) {
+    std::unique_lock<std::mutex> lk(s.m);
+    const unsigned long mine = s.next++;
+    s.cv.wait(lk, [&] { return s.serving == mine && s.used + held <= cap; });
+    s.serving++;
+    s.used += held;
+    s.cv.notify_all();
+  }
+  ~SlotHold() {
+    std::lock_guard<std::mutex> lk(s.m);
+    s.used -= held;
+    s.cv.notify_all();
+  }
+
+ private:
+  Slots &s;
+  const long held;
+};
+
 constexpr int kSyncStride = 32;                     // words between the groups' counters: 128 bytes
 
 constexpr long long kDefaultWait = 20000000000LL;   // cycles (about 10 s at 2 GHz)
@@ -251,7 +288,7 @@ __device__ __forceinline__ void group_cg(const BLat &L, double *part_pq, double 
 // CLOV = 1: A_oo^-1 from the packed inverse blocks and A_ee from the clover term (d <= 6);
 // CLOV = 0: no clover term, A_oo = 1 and the (4+m)^2 diagonal.
 template <int D, int CLOV>
-__global__ void __launch_bounds__(kThreads, 3) k_cg_batch(const __grid_constant__ BArgs args, double *part_pq,
+__global__ void __launch_bounds__(kThreads, kPerSM) k_cg_batch(const __grid_constant__ BArgs args, double *part_pq,
                                                        double *part_rr, unsigned *sync, int *err, BOut *out,
                                                        long long limit) {
   int li = 0;
@@ -276,14 +313,30 @@ void launch_batch(int grid, cudaStream_t s, const BArgs &a, double *part_pq, dou
   YG_LAUNCHED();
 }
 
-template <int D, int CLOV>
-int resident_blocks() {
-  int dev = 0, sms = 0, per = 0;
+int sm_count() {
+  int dev = 0, sms = 0;
   YG_CUDA(cudaGetDevice(&dev));
   YG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  YG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cg_batch<D, CLOV>, kThreads, 0));
-  return sms * per;
+  return sms;
 }
+
+template <int D, int CLOV>
+int resident_blocks() {
+  int per = 0;
+  YG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cg_batch<D, CLOV>, kThreads, 0));
+  return sm_count() * per;
+}
+
+// one device buffer: partials, barrier counters, error flag, results
+struct WorkLayout {
+  size_t sync, err, out, bytes;
+  WorkLayout(int n, int grid) {
+    sync = (2 * sizeof(double) * grid + 127) / 128 * 128;
+    err = sync + sizeof(unsigned) * kSyncStride * n;
+    out = err + 16;
+    bytes = out + sizeof(BOut) * n;
+  }
+};
 
 // the representation dimensions of the persistent batch: SU(2) fundamental (2), SU(3)
 // fundamental and SU(2) adjoint (3), SU(4) fundamental (4), SU(3) sextet and SU(4)
@@ -311,6 +364,12 @@ bool batch_eligible(int n, Lattice *const *L, const yg_inv_par *par) {
     if (l.p.bc == YG_BC_OPEN || l.p.bc == YG_BC_SF) return false;   // spinor boundary slices
   }
   return true;
+}
+
+void persistent_prepare(Lattice &L) {
+  int grid_max = 0;
+  YG_BATCH_D(L.d, L.p.clover, grid_max = resident_blocks<BD, BC>());
+  L.cg_work.alloc(WorkLayout(1, grid_max).bytes);
 }
 
 // The cg_inverter prologue on every lattice (cg.cpp:134-150: r = b - A x, p = r, |b|^2, |r|^2)
@@ -371,30 +430,26 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
   }
   const int grid = b0;
   if (grid > grid_max) throw Error(YG_ERR_ARG, "block groups exceed the resident grid");
-  // one device buffer: partials, barrier counters, error flag, results
-  const size_t off_sync = (2 * sizeof(double) * grid + 127) / 128 * 128;
-  const size_t off_err = off_sync + sizeof(unsigned) * kSyncStride * n;
-  const size_t off_out = off_err + 16;
-  const size_t bytes = off_out + sizeof(BOut) * n;
-  L[0]->cg_work.alloc(bytes);            // kept: an allocation would synchronise the device on every solve
+  const WorkLayout lay(n, grid);
+  L[0]->cg_work.alloc(lay.bytes);        // kept: an allocation would synchronise the device on every solve
   char *base = L[0]->cg_work.as<char>();
   cudaStream_t s = L[0]->stream;
   int err = 0, step = launch_iters(vol);
   bool more = true;
   std::vector<BOut> res(n);
-  std::lock_guard<std::mutex> one(g_persistent[L[0]->device % kMaxDevices]);
   try {
     const long long limit = wait_cycles > 0 ? wait_cycles : kDefaultWait;
     double *part = reinterpret_cast<double *>(base);
     while (more && !err) {
       for (int i = 0; i < n; i++) h[i].it1 = h[i].it0 + step;
-      YG_CUDA(cudaMemsetAsync(base, 0, bytes, s));
+      SlotHold hold(L[0]->device, grid, (long)kPerSM * sm_count());
+      YG_CUDA(cudaMemsetAsync(base, 0, lay.bytes, s));
       YG_BATCH_D(d, clov, launch_batch<BD, BC>(grid, s, args, part, part + grid,
-                                               reinterpret_cast<unsigned *>(base + off_sync),
-                                               reinterpret_cast<int *>(base + off_err),
-                                               reinterpret_cast<BOut *>(base + off_out), limit));
-      YG_CUDA(cudaMemcpyAsync(res.data(), base + off_out, sizeof(BOut) * n, cudaMemcpyDeviceToHost, s));
-      YG_CUDA(cudaMemcpyAsync(&err, base + off_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+                                               reinterpret_cast<unsigned *>(base + lay.sync),
+                                               reinterpret_cast<int *>(base + lay.err),
+                                               reinterpret_cast<BOut *>(base + lay.out), limit));
+      YG_CUDA(cudaMemcpyAsync(res.data(), base + lay.out, sizeof(BOut) * n, cudaMemcpyDeviceToHost, s));
+      YG_CUDA(cudaMemcpyAsync(&err, base + lay.err, sizeof(int), cudaMemcpyDeviceToHost, s));
       YG_CUDA(cudaStreamSynchronize(s));
       more = false;
       for (int i = 0; i < n; i++) {

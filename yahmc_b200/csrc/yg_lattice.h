@@ -209,6 +209,8 @@ int cg(Lattice &L, const yg_inv_par &par, double *x, double *b, int *iters);
 // cg on several lattices at once, one host thread and the lattice's own stream each (yg_solvers.cu)
 int cg_lattices(int n, Lattice *const *L, const yg_inv_par *par, double *const *xs, double *const *bs, int *iters,
                 long long wait_cycles = 0, int *persistent = nullptr);
+// the buffer of a solve of one lattice, so that no host thread allocates while others' solves run
+void persistent_prepare(Lattice &L);
 bool batch_eligible(int n, Lattice *const *L, const yg_inv_par *par);
 int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, double *const *xs, double *const *bs,
                            int *iters, long long wait_cycles);

@@ -91,9 +91,14 @@ static int cg_launches(Lattice &L, const yg_inv_par &par, double *x, double *b, 
 //   d = 2: 16^4 93 / 45;  d = 6: 8^4 139 / 61, 16^4 309 / 442
 constexpr long kPersistentColours = 100000;     // even sites times d
 
+static bool takes_persistent(Lattice &L, const yg_inv_par &par) {
+  Lattice *l = &L;
+  return L.Vh * L.d <= kPersistentColours && batch_eligible(1, &l, &par);
+}
+
 int cg(Lattice &L, const yg_inv_par &par, double *x, double *b, int *iters) {
   Lattice *l = &L;
-  if (L.Vh * L.d > kPersistentColours || !batch_eligible(1, &l, &par)) return cg_launches(L, par, x, b, iters);
+  if (!takes_persistent(L, par)) return cg_launches(L, par, x, b, iters);
   const int st = cg_lattices_persistent(1, &l, &par, &x, &b, iters, 0);
   if (st == YG_NONFINITE) throw Error(YG_NONFINITE, "non-finite value in cg");
   if (st == YG_TIMEOUT) throw Error(YG_TIMEOUT, "a barrier wait of the persistent CG ran out");
@@ -104,11 +109,17 @@ int cg(Lattice &L, const yg_inv_par &par, double *x, double *b, int *iters) {
 // A small lattice's CG is bound by kernel and reduction latency and leaves most of the GPU
 // idle.  Hphi_sq solves on even-odd lattices of one representation dimension d (2, 3, 4, 6;
 // all with or all without a clover term; no open/SF boundaries) run as one persistent kernel
-// (yg_batch.cu); any other mix runs each lattice's single-lattice cg in its own host thread
-// on the lattice's own stream, so the solves overlap on the device.  Iteration counts are
-// those of one-at-a-time calls (the persistent kernel's reductions add in another order, so
-// a count can differ by one where |r|^2 lands within rounding of the stopping threshold).
+// (yg_batch.cu); any other mix runs each lattice's solve in its own host thread on the lattice's own
+// stream, so the solves overlap on the device: persistent ones as far as they fit together, or, when
+// the lattices are more than kSharedColours in all, launch by launch, which fills the device better.
+// us for one lattice with open boundaries and n - 1 antiperiodic ones, d = 3, 60 iterations, persistent /
+// launches: 8^4 n = 8 6750 / 8160, n = 16 (98304 colours) 9640 / 12060; 12^4 n = 4 (124416) 8900 / 9630,
+// n = 8 (248832) 13590 / 12570, n = 16 24380 / 20850.  Iteration counts are those of one-at-a-time calls
+// (reductions add in another order on the other path, so a count can differ by one where |r|^2 lands
+// within rounding of the stopping threshold).
 // Returns the worst status; *persistent (when given) tells which path ran.
+constexpr long kSharedColours = 150000;         // even sites times d, summed over the lattices
+
 int cg_lattices(int n, Lattice *const *L, const yg_inv_par *par, double *const *xs, double *const *bs, int *iters,
                 long long wait_cycles, int *persistent) {
   if (n < 1 || n > 64) throw Error(YG_ERR_ARG, "1..64 lattices");
@@ -125,8 +136,13 @@ int cg_lattices(int n, Lattice *const *L, const yg_inv_par *par, double *const *
   if (batch) return cg_lattices_persistent(n, L, par, xs, bs, iters, wait_cycles);
   // the scratch fields the solves use, allocated here: a cudaMalloc inside the threads would
   // synchronise the device while the other lattices' solves run
-  for (int i = 0; i < n; i++)
+  long colours = 0;
+  for (int i = 0; i < n; i++) colours += L[i]->Vh * L[i]->d;
+  const bool share = colours <= kSharedColours;
+  for (int i = 0; i < n; i++) {
     for (int k = 1; k <= 5; k++) L[i]->scratch_field(k);
+    if (share && takes_persistent(*L[i], par[i])) persistent_prepare(*L[i]);
+  }
   int dev = 0;
   YG_CUDA(cudaGetDevice(&dev));
   std::vector<int> st(n, YG_OK);
@@ -137,7 +153,7 @@ int cg_lattices(int n, Lattice *const *L, const yg_inv_par *par, double *const *
     th.emplace_back([&, i] {
       try {
         YG_CUDA(cudaSetDevice(dev));
-        st[i] = cg(*L[i], par[i], xs[i], bs[i], &iters[i]);
+        st[i] = (share ? cg : cg_launches)(*L[i], par[i], xs[i], bs[i], &iters[i]);
       } catch (...) {
         err[i] = std::current_exception();
       }
