@@ -18,7 +18,7 @@
 // with a barrier of the group after each phase.  Hphi is Hermitian on these lattices (no open or
 // SF slices), so <p, Hphi_sq p> = |Hphi p|^2 and alpha is known before the second Hphi ends, which
 // leaves five barriers an iteration and no pass over q.  The operator steps are the FP64 Schur
-// steps of the single-lattice path (yg_dirac_impl.cuh: four lanes a site up to kQuadSites) with
+// steps of the single-lattice path (yg_dirac_impl.cuh: a thread or four lanes a site) with
 // ordinary loads for the fields, which the kernel also writes.  The scalars are the reference's:
 // alpha = rr / <p,q>, beta = rr_new / rr, stop when rr_new < prec |b|^2, iteration count as
 // cg_inverter's.  Reductions are deterministic: one partial per block, which every block of the
@@ -385,8 +385,15 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
   BArgs args{};
   args.n = n;
   BLat *h = args.l;
-  long vol = 0;
-  for (int i = 0; i < n; i++) vol += L[i]->Vh;
+  // Four lanes a site only where every lattice is small: beside a larger one, whose group decides the time,
+  // they take multiprocessors from it.  8^4 + 12^4 + 16^4, 60 iterations, four lanes at 8^4 / a thread a
+  // site: d = 2 4190 / 2885 us, d = 3 7450 / 6790, d = 4 11230 / 10375; all small: 16 x 4^4 d = 3 2163 /
+  // 2935, 4 x 8^4 d = 4 2150 / 3500.
+  long vol = 0, largest = 0;
+  for (int i = 0; i < n; i++) {
+    vol += L[i]->Vh;
+    largest = std::max(largest, (long)L[i]->Vh);
+  }
   int grid_max = 0;
   YG_BATCH_D(d, clov, grid_max = resident_blocks<BD, BC>());
   if (grid_max < n) throw Error(YG_ERR_ARG, "more lattices than resident blocks");
@@ -421,7 +428,7 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
     // one block each, the others in proportion to the even volume (so that all shares together fit the
     // resident grid), and no more than the passes over the sites need (fewer blocks make a cheaper barrier)
     const long share = 1 + (grid_max - n) * (long)l.Vh / vol;
-    b.quad = d > kSiteMaxD || l.Vh <= kQuadSites;
+    b.quad = d > kSiteMaxD || largest <= kQuadSites;
     const long tiles = nblk(l.Vh, b.quad ? kThreads / 4 : kThreads), passes = (tiles + share - 1) / share;
     b.nb = (int)((tiles + passes - 1) / passes);
     b.b0 = b0;
