@@ -110,3 +110,13 @@ def test_network_on_ragged_tiles(channels):
     assert abs(loss - lo) < 2e-2 * lo
     for g, h in zip(grads, go):
         assert rel(g, h) < 2e-2
+
+
+@pytest.mark.parametrize("name,dims", [("su4_asym_ap", BELOW), ("su3_adj_ap", BELOW), ("su4_sym_ap", BELOW),
+                                       ("su4_sym_ap", (10, 10, 10, 12)), ("su4_adj_ap", (2, 4, 4, 6))])
+def test_clover_term(name, dims):
+    """A warp per plane up to d = 8 (blocks of 32 sites, the last one ragged), a thread a site above, with
+    leaves as chains (d = 10 below 10000 sites) or as pairs of products."""
+    lat, O, rng = make_pair(name, dims, seed=25)
+    assert rel(lat.clover_term(), O.cl_term, floor=1.0) < TOL
+    assert rel(lat.repr_links(), O.links) < TOL

@@ -9,6 +9,8 @@
 
 namespace yg {
 
+void check_cuda(cudaError_t e, const char *what);      // throws (yg_lattice.h)
+
 // CLOVINV applies the explicit FP32 inverse, CLOVPK the packed Hermitian FP64 inverse
 enum { EPI_PLAIN = 0, EPI_CLOVINV = 1, EPI_CLOVADD = 2, EPI_AXPY = 3, EPI_CLOVPK = 4 };
 

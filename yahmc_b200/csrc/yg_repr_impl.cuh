@@ -127,7 +127,7 @@ __global__ void k_represent(double2 *links, double *real, const double2 *fund, G
 template <int NC, int D>
 __device__ __forceinline__ void clover_leaves(double2 (&out)[D * D], const double2 *fund, const Geom &g, const int c[4],
                                               int id, int mu, int nu, const double2 *basis, int rep) {
-  _Pragma(YG_STR(unroll (D <= 4 ? 64 : 1)))
+  _Pragma(YG_STR(unroll (D <= 4 ? 64 : 8)))
   for (int k = 0; k < D * D; k++) out[k] = make_double2(0, 0);
   int cc[4];
   const int fm = neighbour(g, c, mu, +1), fn = neighbour(g, c, nu, +1);
@@ -166,9 +166,92 @@ __device__ __forceinline__ void clover_leaves(double2 (&out)[D * D], const doubl
     } else {
       double2 R[D * D];
       represent_one<NC, D>(R, X, basis, rep);
-      _Pragma(YG_STR(unroll (D <= 4 ? 64 : 1)))
+      _Pragma(YG_STR(unroll (D <= 4 ? 64 : 8)))
       for (int k = 0; k < D * D; k++) out[k] = cadd(out[k], R[k]);
     }
+  }
+}
+
+template <int N>
+__device__ __forceinline__ void rk_mm(double2 (&c)[N * N], const double2 (&a)[N * N], const double2 (&b)[N * N]) {
+#pragma unroll
+  for (int i = 0; i < N; i++)
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      double2 s = make_double2(0, 0);
+#pragma unroll
+      for (int k = 0; k < N; k++) cfma(s, a[i * N + k], b[k * N + j]);
+      c[i * N + j] = s;
+    }
+}
+
+// c = a b^dag
+template <int N>
+__device__ __forceinline__ void rk_mmd(double2 (&c)[N * N], const double2 (&a)[N * N], const double2 (&b)[N * N]) {
+#pragma unroll
+  for (int i = 0; i < N; i++)
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      double2 s = make_double2(0, 0);
+#pragma unroll
+      for (int k = 0; k < N; k++) cfma(s, a[i * N + k], cconj(b[j * N + k]));
+      c[i * N + j] = s;
+    }
+}
+
+// c = a^dag b
+template <int N>
+__device__ __forceinline__ void rk_mdm(double2 (&c)[N * N], const double2 (&a)[N * N], const double2 (&b)[N * N]) {
+#pragma unroll
+  for (int i = 0; i < N; i++)
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      double2 s = make_double2(0, 0);
+#pragma unroll
+      for (int k = 0; k < N; k++) cfmac(s, a[k * N + i], b[k * N + j]);
+      c[i * N + j] = s;
+    }
+}
+
+// The same with the links of a leaf multiplied in pairs: for d >= 10, where the leaf sums live in local
+// memory either way
+template <int NC, int D>
+__device__ void clover_leaves_tree(double2 (&out)[D * D], const double2 *fund, const Geom &g, const int c[4], int id,
+                              int mu, int nu, const double2 *basis, int rep) {
+  double2 A[NC * NC], B[NC * NC], P[NC * NC], Q[NC * NC], R[D * D];
+  for (int k = 0; k < D * D; k++) out[k] = make_double2(0, 0);
+  int cc[4];
+#pragma unroll 1
+  for (int leaf = 0; leaf < 4; leaf++) {
+    if (leaf == 0) {         // U(x,mu) U(x+mu,nu) [U(x,nu) U(x+nu,mu)]^dag
+      int a = neighbour(g, c, mu, +1), b = neighbour(g, c, nu, +1);
+      rk_load<NC>(A, fund, g, id, mu); rk_load<NC>(B, fund, g, a, nu); rk_mm<NC>(P, A, B);
+      rk_load<NC>(A, fund, g, id, nu); rk_load<NC>(B, fund, g, b, mu); rk_mm<NC>(Q, A, B);
+      rk_mmd<NC>(A, P, Q);
+    } else if (leaf == 1) {  // U(x,nu) [U(x-mu,nu) U(x-mu+nu,mu)]^dag U(x-mu,mu)
+      int a = neighbour(g, c, mu, -1);
+      coords_of(g, a, cc);
+      int b = neighbour(g, cc, nu, +1);
+      rk_load<NC>(A, fund, g, a, nu); rk_load<NC>(B, fund, g, b, mu); rk_mm<NC>(Q, A, B);
+      rk_load<NC>(A, fund, g, id, nu); rk_mmd<NC>(P, A, Q);
+      rk_load<NC>(B, fund, g, a, mu); rk_mm<NC>(A, P, B);
+    } else if (leaf == 2) {  // [U(x-mu-nu,nu) U(x-mu,mu)]^dag U(x-mu-nu,mu) U(x-nu,nu)
+      int a = neighbour(g, c, mu, -1), b = neighbour(g, c, nu, -1);
+      coords_of(g, a, cc);
+      int ci = neighbour(g, cc, nu, -1);
+      rk_load<NC>(A, fund, g, ci, nu); rk_load<NC>(B, fund, g, a, mu); rk_mm<NC>(Q, A, B);
+      rk_load<NC>(A, fund, g, ci, mu); rk_mdm<NC>(P, Q, A);
+      rk_load<NC>(B, fund, g, b, nu); rk_mm<NC>(A, P, B);
+    } else {                 // U(x-nu,nu)^dag U(x-nu,mu) U(x-nu+mu,nu) U(x,mu)^dag
+      int a = neighbour(g, c, nu, -1);
+      coords_of(g, a, cc);
+      int b = neighbour(g, cc, mu, +1);
+      rk_load<NC>(A, fund, g, a, nu); rk_load<NC>(B, fund, g, a, mu); rk_mdm<NC>(P, A, B);
+      rk_load<NC>(B, fund, g, b, nu); rk_mm<NC>(Q, P, B);
+      rk_load<NC>(B, fund, g, id, mu); rk_mmd<NC>(A, Q, B);
+    }
+    represent_one<NC, D>(R, A, basis, rep);
+    for (int k = 0; k < D * D; k++) out[k] = cadd(out[k], R[k]);
   }
 }
 
@@ -191,11 +274,14 @@ __device__ __forceinline__ void clover_entry(double2 (&A)[4], const double2 (&ij
   A[3] = make_double2(-csw * (c_re + d_re), -csw * (c_im + d_im));
 }
 
-// The clover term for d <= 4: a block takes 32 sites with one warp per plane, whose leaf sums
+// The clover term for d <= 8: a block takes 32 sites with one warp per plane, whose leaf sums
 // meet in shared memory, where one thread a site kept all six in local memory (1.1 kB a thread
-// for d = 3, indexed by the plane).  SU(3) 32 x 16^3: 188 us, 282 before (cold caches).
+// for d = 3, indexed by the plane).  SU(3) 32 x 16^3: 188 us, 282 before (cold caches).  Represent + clover
+// term, a thread a site / this: sextet (d = 6) 8^4 483 / 148 us, 16^4 1267 / 1191; SU(4) antisymmetric
+// (d = 6) 8^4 751 / 178, 16^4 2098 / 2064; d = 8 8^4 743 / 196, 12^4 1040 / 788.  SU(4) at d = 6 and
+// d = 8 take the registers of one block an SM (with two, d = 6 of SU(4) spilled: 16^4 3775).
 template <int NC, int D>
-__global__ void __launch_bounds__(192, 2) k_clover_term_planes(double2 *cl, const double2 *fund, Geom g, const double2 *basis,
+__global__ void __launch_bounds__(192, (D <= 4 || (D == 6 && NC == 3) ? 2 : 1)) k_clover_term_planes(double2 *cl, const double2 *fund, Geom g, const double2 *basis,
                                                             int rep, double csw_in) {
   constexpr int DD = D * D;
   extern __shared__ __align__(16) unsigned char leaf_smem[];
@@ -227,8 +313,11 @@ __global__ void __launch_bounds__(192, 2) k_clover_term_planes(double2 *cl, cons
   }
 }
 
-// The same for larger d, one thread a site
-template <int NC, int D>
+// The same for larger d, one thread a site, whose leaf sums (24 kB at d = 15) travel through L2.
+// TREE: leaves as pairs of products.  represent + clover term, chains / pairs: d = 10 4^4 1508 / 1677 us,
+// 8^4 1540 / 1709, 12^4 2440 / 2303, 16^4 5876 / 5225; d = 15 4^4 3628 / 3415, 12^4 6160 / 5140.
+constexpr int kLeafPairSites = 10000;      // d = 10: between 8^4 and 12^4
+template <int NC, int D, bool TREE>
 __global__ void k_clover_term(double2 *cl, const double2 *fund, Geom g, const double2 *basis, int rep, double csw_in) {
   int id = blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= g.V) return;
@@ -242,7 +331,10 @@ __global__ void k_clover_term(double2 *cl, const double2 *fund, Geom g, const do
   const int pm[6][2] = {{0, 1}, {0, 2}, {0, 3}, {1, 2}, {1, 3}, {2, 3}};
   double2 tmp[6][D * D];
 #pragma unroll 1
-  for (int q = 0; q < 6; q++) clover_leaves<NC, D>(tmp[q], fund, g, c, id, pm[q][0], pm[q][1], basis, rep);
+  for (int q = 0; q < 6; q++) {
+    if constexpr (TREE) clover_leaves_tree<NC, D>(tmp[q], fund, g, c, id, pm[q][0], pm[q][1], basis, rep);
+    else clover_leaves<NC, D>(tmp[q], fund, g, c, id, pm[q][0], pm[q][1], basis, rep);
+  }
   for (int i = 0; i < D; i++)
     for (int j = 0; j < D; j++) {
       double2 ij[6], ji[6], A[4];
@@ -272,10 +364,18 @@ void RK<NC, D>::represent(double2 *links, double *real, const double2 *fund, Geo
 template <int NC, int D>
 void RK<NC, D>::clover_term(double2 *cl, const double2 *fund, Geom g, const double2 *basis, int rep, double csw,
                             cudaStream_t s) {
-  if constexpr (D <= 4)        // six planes of d x d entries for 32 sites in shared memory: 48 kB at d = 4
-    k_clover_term_planes<NC, D><<<nblk(g.V, 32), 192, sizeof(double2) * 6 * D * D * 32, s>>>(cl, fund, g, basis, rep, csw);
-  else
-    k_clover_term<NC, D><<<nblk(g.V, 64), 64, 0, s>>>(cl, fund, g, basis, rep, csw);
+  if constexpr (D <= 8) {      // six planes of d x d entries for 32 sites in shared memory: 192 kB at d = 8
+    constexpr int smem = sizeof(double2) * 6 * D * D * 32;
+    if (smem > 48 * 1024)
+      check_cuda(cudaFuncSetAttribute(k_clover_term_planes<NC, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+                 "clover term shared memory");
+    k_clover_term_planes<NC, D><<<nblk(g.V, 32), 192, smem, s>>>(cl, fund, g, basis, rep, csw);
+  } else {
+    if (D == 10 && g.V < kLeafPairSites)
+      k_clover_term<NC, D, D != 10><<<nblk(g.V, 64), 64, 0, s>>>(cl, fund, g, basis, rep, csw);
+    else
+      k_clover_term<NC, D, true><<<nblk(g.V, 64), 64, 0, s>>>(cl, fund, g, basis, rep, csw);
+  }
 }
 
 }  // namespace yg
