@@ -120,3 +120,39 @@ def test_clover_term(name, dims):
     lat, O, rng = make_pair(name, dims, seed=25)
     assert rel(lat.clover_term(), O.cl_term, floor=1.0) < TOL
     assert rel(lat.repr_links(), O.links) < TOL
+
+
+@pytest.mark.parametrize("name,dims", [
+    ("su2_asym_ap", (16, 12, 12, 12)), ("su2_fund_ap", BELOW), ("su3_fund_ap", (4, 4, 4, 4)),
+    ("su3_fund_ap", (14, 12, 12, 12)), ("su3_fund_ap", (16, 12, 12, 12)),
+    ("su4_fund_ap", BELOW), ("su4_fund_ap", (16, 14, 12, 12)),
+    ("su3_sym_ap", BELOW), ("su3_sym_ap", (16, 14, 12, 12)),
+    ("su3_adj_ap", BELOW), ("su4_sym_ap", BELOW), ("su4_adj_ap", (2, 4, 4, 6))])
+def test_fermion_forces_one_and_several_poles(name, dims):
+    """The hopping force of one pole and of three (with and without the pole loop; the spinors of a pole
+    at once or in pairs), and the clover force's three splits (warps on small lattices, a thread a site or
+    per site and slot above), on both sides of the changes at 10000, 25000 and 30000 sites.  The large
+    lattices compare a call of three poles with the oracle's sum on a third of the work: three calls of one
+    pole must give the same, and one of them is the oracle's."""
+    lat, O, rng = make_pair(name, dims, seed=26)
+    fields_ = [source(O, rng) for _ in range(3)]
+    dev = [lat.field(f) for f in fields_]
+    w = (0.7, -0.2, 0.35)
+    first = None
+    lat.zero_momenta()
+    lat.begin_fermion_force()
+    for f, c in zip(dev, w):
+        lat.wilson_fermion_force_q(0.1, -0.5, c, f)
+        if first is None:
+            first = lat.clover_force().copy(), lat.momenta().copy()
+    O.mom[:] = 0
+    O.begin_fermion_force()
+    O.wilson_fermion_force_q(0.1, -0.5, w[0], fields_[0].copy())
+    assert rel(first[0], O.cl_force, floor=1.0) < TOL
+    assert rel(first[1], O.mom, floor=1.0) < TOL
+    one = lat.clover_force().copy(), lat.momenta().copy()
+    lat.zero_momenta()
+    lat.begin_fermion_force()
+    lat.wilson_fermion_force_q_multi(0.1, -0.5, list(w), dev)
+    assert rel(lat.clover_force(), one[0], floor=1.0) < TOL
+    assert rel(lat.momenta(), one[1], floor=1.0) < TOL

@@ -100,7 +100,8 @@ __device__ __forceinline__ double gen_trace(const double2 (&m)[D * D], const dou
 
 // av[a] += coeff/(-TF) * Re tr(iT[a] m)   (algebra_project, suNa.cpp:91-111), TF = 2.  TRACE = false
 // leaves the unrolling to the compiler, which is faster for large matrices in local memory: clover force of
-// d = 8 12^4 28.6 ms, 30.0 with rolled loops; d = 15 8^4 60.6, 66.5
+// d = 8 12^4 28.6 ms, 30.0 with rolled loops; d = 15 8^4 60.6, 66.5 (the hopping force of d = 8, and of
+// d = 10 with several poles, is faster with them: 12^4 12 poles d = 8 4.0 ms / 5.2, d = 10 7.7 / 10.6)
 template <int D, bool TRACE = (D <= 6)>
 __device__ __forceinline__ void project_add(double *mom, const double2 (&m)[D * D], const double2 *gens, int ng,
                                             double coeff) {
@@ -153,10 +154,15 @@ __device__ __forceinline__ void dag(double2 (&c)[D * D], const double2 (&a)[D * 
 
 // X <- M X (DAG: M^dag X) for the matrix M of record (id, slot), in place column by column: the
 // chains of products below are written as such left multiplications, so that a thread holds the
-// running product, one sum and one loaded matrix, and d = 3 stays within 168 registers
+// running product, one sum and one loaded matrix (d = 3: 168 registers and 0.3 to 0.6 kB of spills).
+// Only with the colour loops unrolled: with rolled loops (d >= 8) nvcc 12.9 compiles a chain that
+// alternates lmul and lmul_add (lmul, lmul_add, lmul on one running product) to wrong results, while
+// each alone, the same source on the host (under the address and undefined-behaviour sanitizers) and a
+// build without the front end's optimizations are right.
 template <int D, bool DAG>
 __device__ __forceinline__ void lmul(double2 (&X)[D * D], const double2 *base, const Geom &g, int id, int slot,
                                      int nslots) {
+  static_assert(D <= 6, "unrolled colour loops only");
   double2 M[D * D];
   asm volatile("" ::: "memory");     // M's loads stay behind the previous product: hoisting them all costs spills
   ld_mat<D>(M, base, g, id, slot, nslots);
@@ -182,6 +188,7 @@ __device__ __forceinline__ void lmul(double2 (&X)[D * D], const double2 *base, c
 template <int D>
 __device__ __forceinline__ void lmul_add(double2 (&t)[D * D], const double2 (&X)[D * D], const double2 *base,
                                          const Geom &g, int id, int slot, int nslots) {
+  static_assert(D <= 6, "unrolled colour loops only");
   double2 M[D * D];
   asm volatile("" ::: "memory");
   ld_mat<D>(M, base, g, id, slot, nslots);
@@ -369,8 +376,16 @@ __global__ void k_hopping_force(double *mom, const __grid_constant__ PoleSet ps,
     scale_spinor<D>(a, ps.w[n]);
     outer_acc<D>(f, s, a);
   }
-  lmul<D, false>(f, U, g, id, mu, 4);
-  project_add<D, true>(mom + (4L * id + mu) * ng, f, itrepr, ng, 1.0);
+  mom += (4L * id + mu) * ng;
+  if constexpr (D <= 6) {
+    lmul<D, false>(f, U, g, id, mu, 4);
+    project_add<D>(mom, f, itrepr, ng, 1.0);
+  } else {
+    double2 u[D * D], m[D * D];
+    ld_mat<D>(u, U, g, id, mu, 4);
+    mat_mul<D>(m, u, f);
+    project_add<D, D == 8 || D == 10>(mom, m, itrepr, ng, 1.0);
+  }
 }
 
 // ---- _compute_clover_force, clover.cpp:170-262 (sites of block 1): coeff times the entries of
