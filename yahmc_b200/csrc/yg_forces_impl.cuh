@@ -350,7 +350,14 @@ __global__ void k_clover_fermion_site(double2 *clf, const double2 *lhs, const do
 // projection is linear, so the result equals the sum of the per-pole forces up to rounding).  The
 // four directions of a site sit in neighbouring lanes and share the loads of its spinors; a warp per
 // direction reads them once each and was 5 to 15 % slower.
-template <int D>
+//
+// ONE: a single pole needs no loop and no weights, which cost 10 to 28 % of it (us, with the loop / this:
+// d = 3 16^4 56.6 / 49.0, d = 4 16^4 129 / 111, d = 10 8^4 575 / 440).  WIDE loads the four spinors of a pole
+// at once, which hides their latency but takes registers: us for 12 poles, narrow / wide: d = 3 8^4 40.2 /
+// 36.7, 12^4 98 / 117, 16^4 290 / 329; d = 4 8^4 58 / 51, 16^4 541 / 479; d = 6 8^4 97 / 108, 16^4 932 / 1054;
+// d = 10 8^4 1620 / 1900; for one pole d = 3 16^4 49 / 53, d = 6 16^4 175 / 169.
+constexpr int kHopWideSites = 10000;        // d <= 3, several poles
+template <int D, bool ONE, bool WIDE>
 __global__ void k_hopping_force(double *mom, const __grid_constant__ PoleSet ps, const double2 *U, Geom g,
                                 const double2 *itrepr, int ng) {
   long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -363,28 +370,43 @@ __global__ void k_hopping_force(double *mom, const __grid_constant__ PoleSet ps,
   YG_UNROLL_DF
   for (int k = 0; k < D * D; k++) f[k] = make_double2(0, 0);
 #pragma unroll 1
-  for (int n = 0; n < ps.n; n++) {
+  for (int n = 0; n < (ONE ? 1 : ps.n); n++) {
     double2 a[4][D], s[4][D];
     ld_spinor64<D>(a, ps.lhs[n], g, fw);
     g5_omg<D>(s, a, mu);
-    ld_spinor64<D>(a, ps.rhs[n], g, id);
-    scale_spinor<D>(a, ps.w[n]);
-    outer_acc<D>(f, s, a);
-    ld_spinor64<D>(a, ps.rhs[n], g, fw);
-    g5_omg<D>(s, a, mu);
-    ld_spinor64<D>(a, ps.lhs[n], g, id);
-    scale_spinor<D>(a, ps.w[n]);
-    outer_acc<D>(f, s, a);
+    if constexpr (WIDE) {
+      double2 b[4][D], q[4][D];
+      ld_spinor64<D>(a, ps.rhs[n], g, fw);
+      g5_omg<D>(q, a, mu);
+      ld_spinor64<D>(a, ps.rhs[n], g, id);
+      ld_spinor64<D>(b, ps.lhs[n], g, id);
+      if (!ONE) {
+        scale_spinor<D>(a, ps.w[n]);
+        scale_spinor<D>(b, ps.w[n]);
+      }
+      outer_acc<D>(f, s, a);
+      outer_acc<D>(f, q, b);
+    } else {
+      ld_spinor64<D>(a, ps.rhs[n], g, id);
+      if (!ONE) scale_spinor<D>(a, ps.w[n]);
+      outer_acc<D>(f, s, a);
+      ld_spinor64<D>(a, ps.rhs[n], g, fw);
+      g5_omg<D>(s, a, mu);
+      ld_spinor64<D>(a, ps.lhs[n], g, id);
+      if (!ONE) scale_spinor<D>(a, ps.w[n]);
+      outer_acc<D>(f, s, a);
+    }
   }
   mom += (4L * id + mu) * ng;
+  const double coeff = ONE ? ps.w[0] : 1.0;
   if constexpr (D <= 6) {
     lmul<D, false>(f, U, g, id, mu, 4);
-    project_add<D>(mom, f, itrepr, ng, 1.0);
+    project_add<D>(mom, f, itrepr, ng, coeff);
   } else {
     double2 u[D * D], m[D * D];
     ld_mat<D>(u, U, g, id, mu, 4);
     mat_mul<D>(m, u, f);
-    project_add<D, D == 8 || D == 10>(mom, m, itrepr, ng, 1.0);
+    project_add<D, D == 8 || (D == 10 && !ONE)>(mom, m, itrepr, ng, coeff);
   }
 }
 
@@ -560,7 +582,13 @@ void DK<D>::clover_fermion_force(double2 *clf, const PoleSet &ps, Geom g, cudaSt
 template <int D>
 void DK<D>::hopping_force(double *mom, const PoleSet &ps, const double2 *U, Geom g, const double2 *itrepr, int ng,
                           cudaStream_t s) {
-  k_hopping_force<D><<<nblk(4L * g.V, 64), 64, 0, s>>>(mom, ps, U, g, itrepr, ng);
+  const int grid = nblk(4L * g.V, 64);
+  if (ps.n == 1)
+    k_hopping_force<D, true, D == 6><<<grid, 64, 0, s>>>(mom, ps, U, g, itrepr, ng);
+  else if (D == 4 || (D <= 3 && g.V <= kHopWideSites))
+    k_hopping_force<D, false, D <= 4><<<grid, 64, 0, s>>>(mom, ps, U, g, itrepr, ng);
+  else
+    k_hopping_force<D, false, false><<<grid, 64, 0, s>>>(mom, ps, U, g, itrepr, ng);
 }
 
 template <int D>
