@@ -294,11 +294,19 @@ __device__ __forceinline__ void clover_slot_row(double2 *clf, const PoleSet &ps,
   }
 }
 
-// Which split: d <= 3 a warp per slot of 32 sites with a constant slot (sigma psi is a renaming of
-// psi's registers); d = 4 and d >= 8, where that spills, a warp per slot and row (blockIdx.y); d = 6
-// one thread a site, slot after slot and pole after pole (k_clover_fermion_site).  us for one pole, a
-// thread a site / this split: d = 3 32 x 16^3 134 / 118; d = 4 16^4 120 / 114; d = 8 12^4 720 / 124; d = 15
-// 8^4 1601 / 114 (d = 6 16^4: 286 a thread a site, 410 a row, 458 a slot).
+// Three splits.  Small lattices, and d >= 8 always: d <= 3 a warp per slot of 32 sites with a constant slot
+// (sigma psi is a renaming of psi's registers), d >= 4, where that spills, a warp per slot and row
+// (blockIdx.y).  Larger lattices, one pole: a thread a site, slot after slot (k_clover_fermion_site).
+// Larger lattices, several poles: as on small ones, d = 4 and 6 a thread per site and slot
+// (k_clover_fermion_slots).  us, operands in L2, warps / a thread a site, one pole:
+//   d = 3 8^4 11 / 31, 12^4 18.4 / 16.6, 16 x 12^3 21.0 / 16.6, 16^4 51.2 / 41.2, 32 x 16^3 132 / 137, 24^4 322 / 311;
+//   d = 1 24^4 20.8 / 16.2; d = 2 16^4 14.6 / 18.6, 24 x 16^3 20.8 / 19.7;
+//   d = 4 8^4 12.4 / 52.7, 16^4 116 / 123, 24 x 16^3 205 / 183;
+//   d = 6 8^4 23 / 119, 12^4 96 / 121, 16 x 12^3 145 / 144, 16^4 419 / 292; d = 8 12^4 125 / 665.
+// 12 poles, warps / a thread per site and slot: d = 4 8^4 58 / 68, 12^4 240 / 253, 16^4 970 / 702; d = 6 4^4 40 / 143,
+// 8^4 134 / 198, 12^4 887 / 861, 16^4 2790 / 2350 (pole after pole a thread a site 3350).
+template <int D> constexpr int kClfSiteOne = D == 2 || D == 4 ? 80000 : 25000;     // sites from which one pole ...
+constexpr int kClfSlotsMany = 30000;                                              // ... and several change over
 template <int D>
 __global__ void __launch_bounds__(192) k_clover_fermion_force(double2 *clf, const __grid_constant__ PoleSet ps, Geom g) {
   const int id = blockIdx.x * 32 + (threadIdx.x & 31), i = blockIdx.y;
@@ -315,6 +323,12 @@ __global__ void __launch_bounds__(192) k_clover_fermion_force(double2 *clf, cons
     case 4: slot(4); break;
     default: slot(5); break;
   }
+}
+
+template <int D>
+__global__ void k_clover_fermion_slots(double2 *clf, const __grid_constant__ PoleSet ps, Geom g) {
+  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (t < 6L * g.V) clover_slot_force<D>(clf, ps, g, (int)(t / 6), (int)(t % 6));
 }
 
 template <int D>
@@ -571,12 +585,19 @@ __global__ void k_clover_force_core_link(double *mom, const double2 *clf, const 
 // ------------------------------------------------------------------ launchers
 template <int D>
 void DK<D>::clover_fermion_force(double2 *clf, const PoleSet &ps, Geom g, cudaStream_t s) {
-  if constexpr (D == 6) {
-    for (int n = 0; n < ps.n; n++)
-      k_clover_fermion_site<D><<<nblk(g.V, 64), 64, 0, s>>>(clf, ps.lhs[n], ps.rhs[n], g, ps.w[n]);
-  } else {
-    k_clover_fermion_force<D><<<dim3(nblk(g.V, 32), D <= 3 ? 1 : D), 192, 0, s>>>(clf, ps, g);
+  if constexpr (D <= 6) {
+    if (ps.n == 1 && g.V > kClfSiteOne<D>) {
+      k_clover_fermion_site<D><<<nblk(g.V, 64), 64, 0, s>>>(clf, ps.lhs[0], ps.rhs[0], g, ps.w[0]);
+      return;
+    }
   }
+  if constexpr (D == 4 || D == 6) {
+    if (ps.n > 1 && g.V > kClfSlotsMany) {
+      k_clover_fermion_slots<D><<<nblk(6L * g.V, 64), 64, 0, s>>>(clf, ps, g);
+      return;
+    }
+  }
+  k_clover_fermion_force<D><<<dim3(nblk(g.V, 32), D <= 3 ? 1 : D), 192, 0, s>>>(clf, ps, g);
 }
 
 template <int D>
