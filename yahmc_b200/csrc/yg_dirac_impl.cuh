@@ -1190,7 +1190,8 @@ static void launch_hop_links(const HopArgs<R> &a, cudaStream_t s) {
   } else {
     using T = RowTile<D, R>;
     if (T::smem > 48 * 1024)
-      cudaFuncSetAttribute(k_hop_rows<D, R, EPI, REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem);
+      check_cuda(cudaFuncSetAttribute(k_hop_rows<D, R, EPI, REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)T::smem), "operator shared memory");
     k_hop_rows<D, R, EPI, REAL><<<nblk(a.n, 32), T::threads, T::smem, s>>>(a);
   }
 }
