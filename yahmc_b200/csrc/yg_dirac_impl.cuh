@@ -645,9 +645,8 @@ __global__ void __launch_bounds__(128) k_hop_quad(HopArgs<R> a) {
 // is bound by HBM and faster (d = 3 32^4: 907 / 1126 us; d = 6 32 x 16^3: 423 / 532 us).
 template <int D, typename R> struct RowTile {
   static constexpr int threads = 32 * D;
-  // directions staged together: all eight, or two passes of four where 8 would leave one block per SM
-  static constexpr int dirs = D <= 6 ? 8 : 4;
-  static constexpr int words = dirs * 2 * D > 4 * D ? dirs * 2 * D : 4 * D;
+  // half spinors of four directions at a time (eight would leave one block per SM), later the 4 d words of a site
+  static constexpr int words = 4 * 2 * D;
   static constexpr size_t smem = sizeof(cplx<R>) * 32 * words;
 };
 
@@ -812,45 +811,25 @@ __device__ __forceinline__ bool hop_rows(const HopArgs<R> &a, int tile, cplx<R> 
     f[mu] = neighbour(g, c, mu, +1);
     b[mu] = neighbour(g, c, mu, -1);
   }
-  if (RowTile<D, R>::dirs == 8) {
-    row_gather<D, R, 0, -1>(sm, 0, i, lane, a.src, g, f[0]);
-    row_gather<D, R, 0, +1>(sm, 1, i, lane, a.src, g, b[0]);
-    row_gather<D, R, 1, -1>(sm, 2, i, lane, a.src, g, f[1]);
-    row_gather<D, R, 1, +1>(sm, 3, i, lane, a.src, g, b[1]);
-    row_gather<D, R, 2, -1>(sm, 4, i, lane, a.src, g, f[2]);
-    row_gather<D, R, 2, +1>(sm, 5, i, lane, a.src, g, b[2]);
-    row_gather<D, R, 3, -1>(sm, 6, i, lane, a.src, g, f[3]);
-    row_gather<D, R, 3, +1>(sm, 7, i, lane, a.src, g, b[3]);
-    __syncthreads();
-    row_apply<D, R, 0, -1>(acc, sm, 0, i, lane, U, g, id);
-    row_apply<D, R, 0, +1>(acc, sm, 1, i, lane, U, g, b[0]);
-    row_apply<D, R, 1, -1>(acc, sm, 2, i, lane, U, g, id);
-    row_apply<D, R, 1, +1>(acc, sm, 3, i, lane, U, g, b[1]);
-    row_apply<D, R, 2, -1>(acc, sm, 4, i, lane, U, g, id);
-    row_apply<D, R, 2, +1>(acc, sm, 5, i, lane, U, g, b[2]);
-    row_apply<D, R, 3, -1>(acc, sm, 6, i, lane, U, g, id);
-    row_apply<D, R, 3, +1>(acc, sm, 7, i, lane, U, g, b[3]);
-  } else {
-    row_gather<D, R, 0, -1>(sm, 0, i, lane, a.src, g, f[0]);
-    row_gather<D, R, 0, +1>(sm, 1, i, lane, a.src, g, b[0]);
-    row_gather<D, R, 1, -1>(sm, 2, i, lane, a.src, g, f[1]);
-    row_gather<D, R, 1, +1>(sm, 3, i, lane, a.src, g, b[1]);
-    __syncthreads();
-    row_apply<D, R, 0, -1>(acc, sm, 0, i, lane, U, g, id);
-    row_apply<D, R, 0, +1>(acc, sm, 1, i, lane, U, g, b[0]);
-    row_apply<D, R, 1, -1>(acc, sm, 2, i, lane, U, g, id);
-    row_apply<D, R, 1, +1>(acc, sm, 3, i, lane, U, g, b[1]);
-    __syncthreads();
-    row_gather<D, R, 2, -1>(sm, 0, i, lane, a.src, g, f[2]);
-    row_gather<D, R, 2, +1>(sm, 1, i, lane, a.src, g, b[2]);
-    row_gather<D, R, 3, -1>(sm, 2, i, lane, a.src, g, f[3]);
-    row_gather<D, R, 3, +1>(sm, 3, i, lane, a.src, g, b[3]);
-    __syncthreads();
-    row_apply<D, R, 2, -1>(acc, sm, 0, i, lane, U, g, id);
-    row_apply<D, R, 2, +1>(acc, sm, 1, i, lane, U, g, b[2]);
-    row_apply<D, R, 3, -1>(acc, sm, 2, i, lane, U, g, id);
-    row_apply<D, R, 3, +1>(acc, sm, 3, i, lane, U, g, b[3]);
-  }
+  row_gather<D, R, 0, -1>(sm, 0, i, lane, a.src, g, f[0]);
+  row_gather<D, R, 0, +1>(sm, 1, i, lane, a.src, g, b[0]);
+  row_gather<D, R, 1, -1>(sm, 2, i, lane, a.src, g, f[1]);
+  row_gather<D, R, 1, +1>(sm, 3, i, lane, a.src, g, b[1]);
+  __syncthreads();
+  row_apply<D, R, 0, -1>(acc, sm, 0, i, lane, U, g, id);
+  row_apply<D, R, 0, +1>(acc, sm, 1, i, lane, U, g, b[0]);
+  row_apply<D, R, 1, -1>(acc, sm, 2, i, lane, U, g, id);
+  row_apply<D, R, 1, +1>(acc, sm, 3, i, lane, U, g, b[1]);
+  __syncthreads();
+  row_gather<D, R, 2, -1>(sm, 0, i, lane, a.src, g, f[2]);
+  row_gather<D, R, 2, +1>(sm, 1, i, lane, a.src, g, b[2]);
+  row_gather<D, R, 3, -1>(sm, 2, i, lane, a.src, g, f[3]);
+  row_gather<D, R, 3, +1>(sm, 3, i, lane, a.src, g, b[3]);
+  __syncthreads();
+  row_apply<D, R, 2, -1>(acc, sm, 0, i, lane, U, g, id);
+  row_apply<D, R, 2, +1>(acc, sm, 1, i, lane, U, g, b[2]);
+  row_apply<D, R, 3, -1>(acc, sm, 2, i, lane, U, g, id);
+  row_apply<D, R, 3, +1>(acc, sm, 3, i, lane, U, g, b[3]);
 #pragma unroll
   for (int s = 0; s < 4; s++) acc[s] = bnd ? mk<R>(0, 0) : cscale(acc[s], a.coeff);
 
