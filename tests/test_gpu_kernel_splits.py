@@ -61,7 +61,8 @@ def test_forces_ragged(name):
 
 
 @pytest.mark.parametrize("name,dims", [("su3_fund_ap", ABOVE), ("su3_fund_ap", BELOW), ("su3_fund_ap_nocl", BELOW),
-                                       ("su3_sym_ap", BELOW), ("su2_fund_ap", (4, 4, 4, 6))])
+                                       ("su3_sym_ap", BELOW), ("su2_fund_ap", (4, 4, 4, 6)), ("su2_fund_ap", ABOVE),
+                                       ("su4_fund_ap", BELOW), ("su4_fund_ap", ABOVE)])
 def test_persistent_cg(name, dims):
     """One lattice per call of cg_inverter: the true residual meets prec and the solution is the
     oracle's CG's (both solve to 1e-11 of |b|; the operator's condition number here is below 1e4)."""

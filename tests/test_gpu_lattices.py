@@ -3,10 +3,12 @@
 Hphi_sq solves on even-odd lattices of one representation dimension (2, 3, 4 or 6), all with
 or all without a clover term and without open/SF boundaries, run as one persistent kernel:
 each lattice's whole cg_inverter loop (cg.cpp:132-202) runs on a group of blocks with
-bounded barriers.  Its reductions add the same terms in another order than the engine's
-single-lattice BLAS, so solutions agree with one-at-a-time calls to rounding (relative 1e-10)
-and iteration counts within one.  Any other mix runs each lattice's single-lattice solve in
-its own host thread and must match one-at-a-time calls bit for bit."""
+bounded barriers.  Small systems of cg_inverter itself take the same kernel, so the persistent
+solves are compared with the recurrence launch by launch (engine operator and BLAS), reached
+through a batch too large for persistent solves: its reductions add the same terms in another
+order, so solutions agree to rounding (relative 1e-10) and iteration counts within one.  Any other
+mix runs each lattice's cg_inverter in its own host thread and must match one-at-a-time calls bit
+for bit."""
 import numpy as np
 import pytest
 
@@ -15,14 +17,36 @@ from tests.helpers import make_pair, source
 pytestmark = pytest.mark.gpu
 
 
-def _setup(case, mass=-0.4, prec=1e-22):
+_filler = []
+
+
+def _launch_by_launch(lat, mass, prec, b, maxiter=0):
+    """cg_inverter's recurrence with one launch per step: the lattice in a batch with one of 165888
+    colours and open boundaries (one iteration), which runs on host threads without the persistent
+    kernel.  Returns the solution on the host and the iteration count."""
+    from yahmc_b200 import Lattice, cg_inverter_lattices
+    if not _filler:
+        big = Lattice((24, 16, 16, 18), bc="open", clover=False)
+        _filler.extend([big, big.field(), big.field(np.ones((big.V, 4, big.d)) + 0j)])
+    x = lat.field()
+    its, rc, path = cg_inverter_lattices([(lat, mass, prec, x, b, maxiter), (_filler[0], 0.5, 1e-30, *_filler[1:], 1)],
+                                         with_path=True)
+    assert path == 0 and rc == 4 and its[1] == 1
+    return lat.download(x), its[0]
+
+
+def _one_call(lat, mass, prec, b):
+    x = lat.field()
+    it = lat.cg_inverter("Hphi_sq", mass, prec, x, b)
+    return lat.download(x), it
+
+
+def _setup(case, mass=-0.4, prec=1e-22, reference=_launch_by_launch):
     solves, refs = [], []
     for k, (name, dims) in enumerate(case):
         lat, O, rng = make_pair(name, dims, seed=90 + k)
         b = lat.field(source(O, rng))
-        x1 = lat.field()
-        it1 = lat.cg_inverter("Hphi_sq", mass, prec, x1, b)
-        refs.append((lat.download(x1), it1))
+        refs.append(reference(lat, mass, prec, b))
         solves.append((lat, mass, prec, lat.field(), b, 0))
     return solves, refs
 
@@ -38,6 +62,9 @@ PERSISTENT = [
     [("su2_fund_ap", (8, 8, 8, 8)), ("su2_fund_ap", (4, 4, 4, 6))],
     [("su4_fund_ap", (8, 4, 4, 4)), ("su4_fund_ap", (4, 4, 4, 4))],
     [("su3_sym_ap", (4, 4, 4, 4)), ("su4_asym_ap", (6, 4, 4, 4))],
+    [("su2_fund_ap", (10, 10, 10, 10)), ("su2_fund_ap", (4, 4, 4, 6))],          # a thread a site
+    [("su4_fund_ap", (8, 10, 10, 12)), ("su4_fund_ap", (4, 4, 4, 4))],
+    [("su3_fund_ap", (16, 16, 16, 14)), ("su3_fund_per", (16, 16, 16, 16))],       # two tiles a block
 ]
 
 
@@ -75,9 +102,9 @@ def test_persistent_batch_maxiter_and_converged_start():
     assert its[0] == 7
     assert abs(its[1] - refs[1][1]) <= 1
     assert its[2] == lat2.cg_inverter("Hphi_sq", m, 1e-16, lat2.field(refs[2][0]), b2) == 0
-    x7 = lat0.field()
-    assert lat0.cg_inverter("Hphi_sq", m, p, x7, b0, maxiter=7) == 7
-    a, c = _even(lat0, x0), _even(lat0, x7)
+    x7, it7 = _launch_by_launch(lat0, m, p, b0, maxiter=7)
+    assert it7 == 7
+    a, c = _even(lat0, x0), x7[:lat0.V // 2]
     assert np.abs(a - c).max() <= 1e-10 * np.abs(c).max()
 
 
@@ -107,7 +134,7 @@ def test_persistent_batch_wait_limit_returns_timeout():
 ])
 def test_threads_equal_sequential(case):
     from yahmc_b200 import cg_inverter_lattices
-    solves, refs = _setup(case)
+    solves, refs = _setup(case, reference=_one_call)
     for _ in range(2):
         for s in solves:
             s[0].spinor_zero(s[3])
@@ -152,12 +179,12 @@ def test_persistent_solve_goes_on_over_several_launches():
     assert np.vdot(r, r).real < 1.1e-14 * np.vdot(b0[:O.Vh], b0[:O.Vh]).real
     # a batch in which one lattice ends in the first launch and one stops at maxiter in the third
     lat2, O2, rng2 = make_pair("su3_fund_ap", (4, 4, 4, 6), seed=24)
-    b2, x2, x2s = lat2.field(source(O2, rng2)), lat2.field(), lat2.field()
-    it2 = lat2.cg_inverter("Hphi_sq", 0.2, 1e-22, x2s, b2)
+    b2, x2 = lat2.field(source(O2, rng2)), lat2.field()
+    x2s, it2 = _launch_by_launch(lat2, 0.2, 1e-22, b2)
     lat.spinor_zero(x)
     its, rc, path = cg_inverter_lattices([(lat, -2.3, 0.0, x, b, 2345), (lat2, 0.2, 1e-22, x2, b2)], with_path=True)
     assert path == 1 and rc == 4 and its[0] == 2345 and abs(its[1] - it2) <= 1
-    got, ref = _even(lat2, x2), _even(lat2, x2s)
+    got, ref = _even(lat2, x2), x2s[:lat2.V // 2]
     assert np.abs(got - ref).max() <= 1e-10 * np.abs(ref).max()
 
 
@@ -225,3 +252,17 @@ def test_host_threads_share_the_device():
     for s in solves:
         assert np.array_equal(_even(s[0], s[2]), _even(s[0], s[3]))
     assert times["threads"] < 0.8 * times["row"], times
+
+
+@pytest.mark.parametrize("name", ["su3_fund_ap", "su4_fund_ap", "su3_sym_ap", "su2_fund_ap", "su3_fund_ap_nocl"])
+def test_launch_by_launch_against_oracle(name):
+    """The recurrence launch by launch, the reference of the tests above, is the oracle's (both solve to
+    1e-11 of |b|; the condition number of the operator is below 1e4)."""
+    lat, O, rng = make_pair(name, (4, 4, 4, 6), seed=77)
+    b0 = source(O, rng)
+    x, it = _launch_by_launch(lat, 0.2, 1e-22, lat.field(b0))
+    xo = O.new_field()
+    ito = O.cg("Hphi_sq", 0.2, 1e-22, xo, b0.copy())
+    ito = ito[0] if isinstance(ito, tuple) else ito
+    assert abs(it - ito) <= 1
+    assert np.abs(x - xo)[:O.Vh].max() < 1e-7 * np.abs(xo[:O.Vh]).max()
