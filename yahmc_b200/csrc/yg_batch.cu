@@ -102,7 +102,10 @@ constexpr int kMore = -1;                           // status of a lattice that 
 // least), against some 20 us for another launch
 int launch_iters(long sites) { return (int)std::max(16L, std::min(1000L, 40000000L / sites)); }
 
-constexpr int kSiteMaxD = 4;                        // d = 6 with a thread a site spills under 168 registers
+// d = 6 always takes four lanes a site, which spill 0.7 kB under 168 registers (d = 4: 0.6 kB, d = 3: 0.1 kB).
+// Batches of 60 iterations, the kernel's first form with a thread a site at all sizes / this: d = 6 8^4 + 12^4
+// 15.6 / 4.6 ms, 8^4 + 12^4 + 16^4 20.6 / 16.5 ms, 8 x 6^4 8.6 / 3.2 ms; d = 4 8^4 + 12^4 + 16^4 13.5 / 10.4 ms.
+constexpr int kSiteMaxD = 4;
 
 struct BLat {
   Geom g;
@@ -110,7 +113,7 @@ struct BLat {
   double2 *x, *r, *p, *t, *o;          // whole-field layout; x, r, p, t even sites, o odd
   int b0, nb;                          // the group's blocks [b0, b0 + nb)
   int quad;                            // four lanes a site instead of one thread
-  int maxiter, it0, it1;               // iterations it0 + 1 .. it1 of this launch; it0 = -1: none, the solve has ended
+  int it0, it1;                        // iterations it0 + 1 .. it1 of this launch; it0 = -1: none, the solve has ended
   double diag, target, rr0;            // diagonal of A_ee, prec |b|^2, |r|^2 after it0 iterations
 };
 
@@ -202,7 +205,6 @@ __device__ __forceinline__ void group_cg(const BLat &L, double *part_pq, double 
   // cg.cpp:151-153: a system solved by its initial guess returns 0 iterations
   while (L.it0 >= 0 && status == YG_OK) {
     ++it;
-    if (L.maxiter > 0 && it > L.maxiter) { it--; status = YG_MAXITER; break; }
 #pragma unroll 1
     for (int half = 0; half < 2; half++) {
       a.src = half ? L.t : L.p;
@@ -420,7 +422,6 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
     b.x = (double2 *)xs[i];
     b.r = (double2 *)r;
     b.p = (double2 *)p;
-    b.maxiter = par[i].maxiter;
     b.target = norm * par[i].prec;
     b.rr0 = rr;
     b.it0 = rr < b.target ? -1 : 0;
@@ -448,7 +449,10 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
     const long long limit = wait_cycles > 0 ? wait_cycles : kDefaultWait;
     double *part = reinterpret_cast<double *>(base);
     while (more && !err) {
-      for (int i = 0; i < n; i++) h[i].it1 = h[i].it0 + step;
+      for (int i = 0; i < n; i++) {
+        h[i].it1 = h[i].it0 + step;
+        if (par[i].maxiter > 0) h[i].it1 = std::min(h[i].it1, par[i].maxiter);
+      }
       SlotHold hold(L[0]->device, grid, (long)kPerSM * sm_count());
       YG_CUDA(cudaMemsetAsync(base, 0, lay.bytes, s));
       YG_BATCH_D(d, clov, launch_batch<BD, BC>(grid, s, args, part, part + grid,
@@ -462,8 +466,9 @@ int cg_lattices_persistent(int n, Lattice *const *L, const yg_inv_par *par, doub
       for (int i = 0; i < n; i++) {
         if (h[i].it0 < 0) continue;
         fin[i] = res[i];
+        if (fin[i].status == kMore && fin[i].iters == par[i].maxiter) fin[i].status = YG_MAXITER;
         h[i].rr0 = res[i].rr;
-        h[i].it0 = res[i].status == kMore ? res[i].iters : -1;
+        h[i].it0 = fin[i].status == kMore ? fin[i].iters : -1;
         more = more || h[i].it0 >= 0;
       }
     }
