@@ -177,6 +177,10 @@ int yg_spinor_mulr_sub_assign(yg_lattice *lat, double *lhs, double v, const doub
 int yg_spinor_mulc_sub_assign(yg_lattice *lat, double *lhs, double re, double im, const double *rhs, int view);
 
 /* ---- inverters (inverter.h:18-22); iterations returned through *iters --- */
+/* Hphi_sq on small even-odd lattices (d = 2, 3, 4, 6, up to 100000 even sites times d, no open/SF
+ * boundaries) iterates in one persistent kernel, at most 1000 iterations a launch.  Should a barrier
+ * wait inside it run out (about 10 s) the call returns YG_TIMEOUT and x holds a partial solve.  Calls of
+ * several host threads on lattices of their own share the device. */
 int yg_cg_inverter(yg_lattice *lat, const yg_inv_par *par, double *x, double *b, int *iters);        /* cg.cpp:132-202 */
 int yg_bicgstab_inverter(yg_lattice *lat, const yg_inv_par *par, double *x, double *b, int *iters);  /* bicgstab.cpp:9-97 */
 int yg_minres_inverter(yg_lattice *lat, const yg_inv_par *par, double *x, double *b, int *iters);    /* minres.cpp:12-117 */
@@ -213,7 +217,7 @@ int yg_cg_inverter_multi(yg_lattice *lat, const yg_inv_par *par, int nrhs, doubl
  * a clover term and without open/SF boundaries, run as ONE persistent cooperative kernel: a
  * group of blocks per lattice, sized by its volume, runs the lattice's whole CG loop on the
  * device with bounded barriers.  Other mixes run a host thread and the lattice's own stream
- * per solve.  Results and iteration counts are those of separate yg_cg_inverter calls (to
+ * per solve, so that they overlap on the device.  Results and iteration counts are those of separate yg_cg_inverter calls (to
  * rounding); returns the worst status.  Every lattice must have been created on the calling
  * thread's current device (YG_ERR_ARG otherwise). */
 int yg_cg_inverter_lattices(int n, yg_lattice *const *lats, const yg_inv_par *pars, double *const *xs,

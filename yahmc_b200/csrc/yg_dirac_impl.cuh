@@ -401,9 +401,13 @@ __global__ void __launch_bounds__(128) k_hop(HopArgs<R> a) {
 //   mu = 0: X,Y = 2,3, ph = 1, 1;  1: 3,2, i, i;  2: 3,2, 1, -1;  3: 2,3, i, -i
 //
 // Taken up to one block of 32 sites per SM.  There a thread per site is a chain of eight rounds of
-// loads on a few SMs: Hphi_sq on 8^4, a thread per site / four lanes: d = 3 37 / 25 us, d = 4 49 / 33,
-// d = 6 86 / 44.  On a full GPU the lanes' shuffles and shorter runs (8 sites, 128 bytes a load) lose:
-// d = 3 on 16^4 60 / 88 us, on 32^4 907 / 1127 us; d = 6 on 32 x 16^3 423 / 504 us.
+// loads on a few SMs; on a full GPU the lanes' shuffles and shorter runs (8 sites, 128 bytes a load) lose.
+// Hphi_sq, us, a thread per site / four lanes, at 2048, 3840, 4800, 6912, 10368, 16800 and 32768 outputs:
+//   d = 2  28.7/24.6  31.3/24.6  30.9/24.6  32.8/24.6  32.7/29.4  32.8/32.8  36.3/49.8
+//   d = 3  35.9/27.7  37.5/27.7  37.9/32.8  37.3/32.8  39.2/41.0  41.0/45.0  53.4/88.1   (32^4: 810 / 1127)
+//   d = 4  48.4/32.8  49.2/32.8  49.2/40.6  49.2/41.0  49.2/49.2  54.1/73.3  111/149
+//   d = 6  83.7/45.1  87.0/45.1  85.9/59.4  89.2/65.4  129/116    186/150    226/292
+// The line is the one at which no d loses; d = 3 crosses at about 8000 outputs, d = 6 not before 16800.
 constexpr int kQuadSites = 148 * 32;
 
 template <typename C>
@@ -642,7 +646,8 @@ __global__ void __launch_bounds__(128) k_hop_quad(HopArgs<R> a) {
 // accumulators where a thread per site keeps 4 d.  For d >= 8, where a thread per site lives in local
 // memory: Hphi_sq, a thread per site / a warp per colour, d = 8 8^4 211 / 66 us, 16^4 562 / 503 us;
 // d = 10 16^4 989 / 766 us; d = 15 8^4 1653 / 168 us, 16^4 2822 / 1416 us.  Up to d = 6 a thread per site
-// is bound by HBM and faster (d = 3 32^4: 907 / 1126 us; d = 6 32 x 16^3: 423 / 532 us).
+// is bound by HBM and faster (d = 3 32^4, before either loaded the clover entries once: 907 / 1126 us; d = 6
+// 32 x 16^3: 423 / 532 us).
 template <int D, typename R> struct RowTile {
   static constexpr int threads = 32 * D;
   // half spinors of four directions at a time (eight would leave one block per SM), later the 4 d words of a site

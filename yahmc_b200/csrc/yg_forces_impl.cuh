@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(256) k_clover_ldl_force(double2 *clf, const do
 // S = U(x-nu,mu)^dag, C = U(x-nu+mu,nu)^dag).  A block takes 32 sites and one direction mu, one
 // warp per nu != mu, and the projected planes are summed in shared memory.  Bound by FP64 latency at
 // 12 warps an SM (168 registers).  SU(3) 32 x 16^3: 459 us, 647 with a thread a link and 13 matrices;
-// d = 6 16^4: 7.9 ms, 14.0.
+// d = 6 16^4: 7.9 ms, 14.0, at 255 registers with 26 kB of spill stores a thread.
 template <int D, bool UP>
 __device__ __forceinline__ void clover_loop(double2 (&t)[D * D], const double2 *clf, const double2 *U, const Geom &g,
                                             int num, int mu, int nu, int x0, int x1, int aid, int sid, int cid, int za,

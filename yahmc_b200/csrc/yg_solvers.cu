@@ -86,9 +86,14 @@ static int cg_launches(Lattice &L, const yg_inv_par &par, double *x, double *b, 
 
 // cg_inverter.  The systems the persistent kernel covers (Hphi_sq with even-odd preconditioning, no
 // open or SF slices, d = 2, 3, 4, 6) iterate wholly on the device while the launches and host round
-// trips of an iteration weigh more than its data; us an iteration, launches / persistent:
-//   d = 3: 4^4 86 / 28, 8^4 85 / 29, 12^4 91 / 61, 16^4 130 / 107, 32 x 16^3 234 / 250, 32^4 1146 / 1300;
-//   d = 2: 16^4 93 / 45;  d = 6: 8^4 139 / 61, 16^4 309 / 442
+// trips of an iteration weigh more than its data; us an iteration, launches / persistent (with clover term):
+//   d = 2: 8^4 74 / 20, 16^4 93 / 35, 24 x 16^3 (98304 colours) 108 / 46, 32 x 16^3 (131072) 115 / 81;
+//   d = 3: 4^4 74 / 24, 8^4 76 / 25, 12^4 92 / 50, 16^4 (98304) 116 / 79, 24 x 16^3 (147456) 153 / 125,
+//          32 x 16^3 (196608) 212 / 217;  SU(2) adjoint 16^4 106 / 80, 24 x 16^3 129 / 124, 32 x 16^3 181 / 217;
+//   d = 4: 8^4 79 / 33, 12^4 108 / 71, 16^3 x 12 (98304) 150 / 153, 16^4 (131072) 174 / 182;
+//   d = 6: 8^4 93 / 51, 12^4 201 / 118, 16 x 12^3 (82944) 240 / 130, 16^3 x 12 (147456) 276 / 236, 16^4 300 / 341.
+// The limit lies where d = 4 meets the launches.  d = 2, 3 and 6 would gain up to 150000 colours from a solve
+// alone, but such a solve fills the device, where launches of several host threads overlap better.
 constexpr long kPersistentColours = 100000;     // even sites times d
 
 static bool takes_persistent(Lattice &L, const yg_inv_par &par) {
