@@ -108,6 +108,7 @@ int yg_lattice_create(const yg_params *p, yg_lattice **out);
 int yg_set_device(int device);
 void yg_lattice_destroy(yg_lattice *lat);
 int yg_lattice_query(const yg_lattice *lat, yg_info *out);
+/* the stream of the lattice's later launches; it stays the caller's and is not destroyed with the lattice */
 int yg_set_stream(yg_lattice *lat, void *cuda_stream);
 int yg_synchronize(yg_lattice *lat);
 const char *yg_last_error(void);

@@ -130,3 +130,26 @@ def test_maxiter_status():
     x, b = lat.field(), lat.field(source(O, rng))
     it = lat.cg_inverter("Hphi_sq", -0.2, 1e-28, x, b, maxiter=3)
     assert it == 3 and lat.last_status == 4
+
+
+def test_callers_stream_outlives_the_lattice():
+    """A stream given with set_stream stays usable after the lattice is closed: the lattice
+    destroys its own stream only."""
+    import torch
+    st = torch.cuda.Stream()
+    lat, O, rng = make_pair("su3_fund_ap", (4, 4, 4, 4), seed=12)
+    src = source(O, rng)
+    lat.set_stream(st.cuda_stream)
+    s, d = lat.field(src), lat.field()
+    lat.Hphi_sq(-0.5, d, s)
+    got = lat.download(d)
+    want = O.new_field()
+    O.Hphi_sq(-0.5, want, src.copy())
+    assert np.abs(got - want).max() < 1e-13 * np.abs(want).max()
+    s.free()
+    d.free()
+    lat.close()
+    with torch.cuda.stream(st):
+        x = torch.ones(1000, device="cuda").sum()
+    st.synchronize()
+    assert x.item() == 1000

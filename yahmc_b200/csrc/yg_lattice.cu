@@ -45,10 +45,10 @@ Lattice::~Lattice() {
   if (sl_hist) cudaFreeHost(sl_hist);
   if (mr_hist) cudaFreeHost(mr_hist);
   for (cudaEvent_t e : sl_ev) if (e) cudaEventDestroy(e);
-  if (stream) {
-    cudaStreamSynchronize(stream);
-    cudaStreamDestroy(stream);
-  }
+  // a stream given to yg_set_stream stays its owner's, who may have destroyed it already
+  if (stream == own_stream) cudaStreamSynchronize(stream);
+  else cudaDeviceSynchronize();
+  if (own_stream) cudaStreamDestroy(own_stream);
   for (DevBuf *b : {&fund, &links, &clover, &ldl, &cl_force, &mom, &tables, &red_partial, &red_result, &links_f,
                     &clover_f, &cinv_f, &sl_links, &sl_clover, &cpk64, &sl_part, &sl_scal, &fund_backup, &sl_cnorm,
                     &mr_work, &mr_scal, &mr_part, &mr_clov, &cg_work, &links_r})
@@ -281,7 +281,8 @@ Lattice *lattice_create(const yg_params &p) {
   try {
     // the lattice's own stream; a blocking stream, so work on the legacy default stream
     // (and events recorded there) still orders with it
-    YG_CUDA(cudaStreamCreateWithFlags(&L->stream, cudaStreamDefault));
+    YG_CUDA(cudaStreamCreateWithFlags(&L->own_stream, cudaStreamDefault));
+    L->stream = L->own_stream;
     YG_CUDA(cudaGetDevice(&L->device));
     L->p = p;
     L->d = d;

@@ -54,7 +54,8 @@ struct Lattice {
   Geom g{};
   int d = 0, nc = 0, ng = 0;
   long V = 0, Vh = 0;
-  cudaStream_t stream = 0;
+  cudaStream_t stream = 0;       // the launches' stream: own_stream, or the one yg_set_stream was given
+  cudaStream_t own_stream = 0;
   int mvm = 0;
   int device = 0;          // the CUDA device the lattice was created on
 
