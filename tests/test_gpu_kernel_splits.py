@@ -124,15 +124,15 @@ def test_clover_term(name, dims):
 
 
 @pytest.mark.parametrize("name,dims", [
-    ("su2_asym_ap", (16, 12, 12, 12)), ("su2_fund_ap", BELOW), ("su3_fund_ap", (4, 4, 4, 4)),
+    ("su2_asym_ap", (24, 16, 16, 14)), ("su2_fund_ap", BELOW), ("su3_fund_ap", (4, 4, 4, 4)),
     ("su3_fund_ap", (14, 12, 12, 12)), ("su3_fund_ap", (16, 12, 12, 12)),
-    ("su4_fund_ap", BELOW), ("su4_fund_ap", (16, 14, 12, 12)),
+    ("su4_fund_ap", BELOW), ("su4_fund_ap", (16, 14, 12, 12)), ("su4_fund_ap", (24, 16, 16, 14)),
     ("su3_sym_ap", BELOW), ("su3_sym_ap", (16, 14, 12, 12)),
     ("su3_adj_ap", BELOW), ("su4_sym_ap", BELOW), ("su4_adj_ap", (2, 4, 4, 6))])
 def test_fermion_forces_one_and_several_poles(name, dims):
     """The hopping force of one pole and of three (with and without the pole loop; the spinors of a pole
     at once or in pairs), and the clover force's three splits (warps on small lattices, a thread a site or
-    per site and slot above), on both sides of the changes at 10000, 25000 and 30000 sites.  The large
+    per site and slot above), on both sides of the changes at 10000 to 80000 sites.  The large
     lattices compare a call of three poles with the oracle's sum on a third of the work: three calls of one
     pole must give the same, and one of them is the oracle's."""
     lat, O, rng = make_pair(name, dims, seed=26)

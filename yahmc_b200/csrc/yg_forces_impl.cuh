@@ -298,15 +298,24 @@ __device__ __forceinline__ void clover_slot_row(double2 *clf, const PoleSet &ps,
 // (sigma psi is a renaming of psi's registers), d >= 4, where that spills, a warp per slot and row
 // (blockIdx.y).  Larger lattices, one pole: a thread a site, slot after slot (k_clover_fermion_site).
 // Larger lattices, several poles: as on small ones, d = 4 and 6 a thread per site and slot
-// (k_clover_fermion_slots).  us, operands in L2, warps / a thread a site, one pole:
-//   d = 3 8^4 11 / 31, 12^4 18.4 / 16.6, 16 x 12^3 21.0 / 16.6, 16^4 51.2 / 41.2, 32 x 16^3 132 / 137, 24^4 322 / 311;
-//   d = 1 24^4 20.8 / 16.2; d = 2 16^4 14.6 / 18.6, 24 x 16^3 20.8 / 19.7;
-//   d = 4 8^4 12.4 / 52.7, 16^4 116 / 123, 24 x 16^3 205 / 183;
-//   d = 6 8^4 23 / 119, 12^4 96 / 121, 16 x 12^3 145 / 144, 16^4 419 / 292; d = 8 12^4 125 / 665.
-// 12 poles, warps / a thread per site and slot: d = 4 8^4 58 / 68, 12^4 240 / 253, 16^4 970 / 702; d = 6 4^4 40 / 143,
-// 8^4 134 / 198, 12^4 887 / 861, 16^4 2790 / 2350 (pole after pole a thread a site 3350).
-template <int D> constexpr int kClfSiteOne = D == 2 || D == 4 ? 80000 : 25000;     // sites from which one pole ...
-constexpr int kClfSlotsMany = 30000;                                              // ... and several change over
+// (k_clover_fermion_slots).  One pole, warps / a thread a site, us with the operands in L2 where they fit,
+// and from DRAM:
+//   d = 1 16^4 9.2/9.0 and 13.2/12.3, 20 x 16^3 10.2/9.0 and 13.1/13.1, 24^4 20.8/16.2;
+//   d = 2 12^4 10.1/12.3 and 15.2/21.4, 16^4 17.3/20.5 and 27.6/37.7, 32 x 16^3 33.7/31.4 and 50.1/56.3, 24^4 112/111;
+//   d = 3 8^4 11/31, 16 x 12^3 23.5/19.4 and 33.8/39.9, 16^4 52.0/41.9 and 70.6/74.7, 20 x 16^3 86/93 and 89/103,
+//         32 x 16^3 132/139, 32 x 20^2 x 16 204/207, 32 x 20^3 250/246, 24^4 320/312, 32 x 24^3 427/414;
+//   d = 4 8^4 12.4/52.7, 16^4 116/123, 24 x 16^3 205/183;
+//   d = 6 8^4 23/119, 12^4 96/121, 16 x 12^3 145/144, 16^4 419/292;  d = 8 12^4 125/665.
+// At d = 3 a thread a site, which reads the spinors once instead of six times, wins where everything stays in
+// L2 (1.25 kB a site, up to 16^4) and, by 2 to 3 %, on the largest lattices; within a whole force the two
+// are equal on 16^4 (operator, this and the hopping force together 194 us).
+// 12 poles, warps / a thread per site and slot: d = 4 8^4 58/68, 12^4 240/253, 16^4 970/702; d = 6 4^4 40/143,
+// 8^4 134/198, 12^4 887/861, 16^4 2790/2350 (pole after pole a thread a site 3350).
+template <int D> constexpr bool clf_site_one(int V) {
+  if (D == 3) return (V > 25000 && V < 75000) || V > 250000;
+  return V > (D == 1 ? 75000 : D == 4 ? 80000 : 25000) && D != 2;
+}
+constexpr int kClfSlotsMany = 30000;        // sites from which several poles take a thread per site and slot
 template <int D>
 __global__ void __launch_bounds__(192) k_clover_fermion_force(double2 *clf, const __grid_constant__ PoleSet ps, Geom g) {
   const int id = blockIdx.x * 32 + (threadIdx.x & 31), i = blockIdx.y;
@@ -586,7 +595,7 @@ __global__ void k_clover_force_core_link(double *mom, const double2 *clf, const 
 template <int D>
 void DK<D>::clover_fermion_force(double2 *clf, const PoleSet &ps, Geom g, cudaStream_t s) {
   if constexpr (D <= 6) {
-    if (ps.n == 1 && g.V > kClfSiteOne<D>) {
+    if (ps.n == 1 && clf_site_one<D>(g.V)) {
       k_clover_fermion_site<D><<<nblk(g.V, 64), 64, 0, s>>>(clf, ps.lhs[0], ps.rhs[0], g, ps.w[0]);
       return;
     }
