@@ -201,9 +201,10 @@ __device__ __forceinline__ void group_cg(const BLat &L, double *part_pq, double 
   e.zero_add_at_boundary = 1;
   unsigned due = 0;
   double rr = L.rr0, alpha = 0.0;
-  int it = L.it0, status = YG_OK;
+  const int it1 = L.it1;
+  int it = L.it0, status = L.it0 >= 0 ? kMore : YG_OK;
   // cg.cpp:151-153: a system solved by its initial guess returns 0 iterations
-  while (L.it0 >= 0 && status == YG_OK) {
+  while (status == kMore) {
     ++it;
 #pragma unroll 1
     for (int half = 0; half < 2; half++) {
@@ -276,9 +277,10 @@ __device__ __forceinline__ void group_cg(const BLat &L, double *part_pq, double 
         }
       }
     }
-    if (status != YG_OK || rr < L.target) break;
-    if (it >= L.it1) status = kMore;
-    else if (!group_sync(cnt, due, nb, err, limit)) status = YG_TIMEOUT;
+    if (status != kMore) break;
+    if (rr < L.target) { status = YG_OK; break; }
+    if (it >= it1) break;
+    if (!group_sync(cnt, due, nb, err, limit)) status = YG_TIMEOUT;
   }
   if (lb == 0 && threadIdx.x == 0) {
     out->iters = it;
