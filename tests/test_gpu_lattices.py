@@ -104,6 +104,7 @@ def test_persistent_batch_maxiter_and_converged_start():
     assert its[2] == lat2.cg_inverter("Hphi_sq", m, 1e-16, lat2.field(refs[2][0]), b2) == 0
     x7, it7 = _launch_by_launch(lat0, m, p, b0, maxiter=7)
     assert it7 == 7
+    assert lat0.cg_inverter("Hphi_sq", m, p, lat0.field(), b0, maxiter=7) == 7
     a, c = _even(lat0, x0), x7[:lat0.V // 2]
     assert np.abs(a - c).max() <= 1e-10 * np.abs(c).max()
 
